@@ -23,7 +23,7 @@ CXX_FLAGS = ["-std=c++20", "-O2", "-fPIC", "-ffp-contract=off", "-Wall", "-Wextr
              "-I/usr/local/cuda/include"]
 
 NVCC_FLAGS = [
-    "-std=c++17", "-O3", "-lineinfo",
+    "-std=c++17", "-O3", "-lineinfo", "--split-compile=0",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC,-O2,-ffp-contract=off",
     "--expt-relaxed-constexpr",

@@ -9,7 +9,10 @@
 // staged once into channel-major rows (one uint8 row per channel, row stride
 // a multiple of 16 bytes); every DM block reuses it.
 //
-// Kernel.  One CTA = a block of DB DMs x a time tile; each warp owns one DM and
+// Kernels.  Large launches run on the tensor cores (dedisperse_mma.cuh); the
+// byte kernel below takes small ones and pinned launch shapes.
+//
+// Byte kernel.  One CTA = a block of DB DMs x a time tile; each warp owns one DM and
 // 1008 consecutive output samples (252 output words of 4 samples).  The CTA
 // streams channel chunks through a ring of 2-4 shared-memory stages: for each
 // channel of a chunk one bulk copy (cp.async.bulk, completion counted in bytes
@@ -443,17 +446,18 @@ __device__ __forceinline__ void bytes_cta(const BytesParams& p, unsigned bx, int
   OutT* out = static_cast<OutT*>(p.out) +
               (static_cast<uint64_t>(dm_local) * p.out_dm_rows +
                static_cast<uint64_t>(group) * p.out_group_rows) * p.out_row_stride;
+  const bool vec = (p.out_row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & (4 * sizeof(OutT) - 1)) == 0;
 #pragma unroll
   for (int m = 0; m < kWords; ++m) {
     const int j = lane + 32 * m;
     if (j >= kOutWords) continue;
     const uint64_t t = t0 + static_cast<uint64_t>(sub) * kWarpSamples + 4ull * j;
     if (t >= p.nout) continue;
-    if (sizeof(OutT) == 4 && t + 4 <= p.nout && (p.out_row_stride & 3) == 0) {
+    if (sizeof(OutT) == 4 && t + 4 <= p.nout && vec) {
       *reinterpret_cast<uint4*>(out + t) =
           make_uint4(acc[(m * 4) * 32 + lane], acc[(m * 4 + 1) * 32 + lane], acc[(m * 4 + 2) * 32 + lane],
                      acc[(m * 4 + 3) * 32 + lane]);
-    } else if (sizeof(OutT) == 1 && t + 4 <= p.nout && (p.out_row_stride & 3) == 0) {
+    } else if (sizeof(OutT) == 1 && t + 4 <= p.nout && vec) {
       *reinterpret_cast<uint32_t*>(out + t) =
           acc[(m * 4) * 32 + lane] | (acc[(m * 4 + 1) * 32 + lane] << 8) | (acc[(m * 4 + 2) * 32 + lane] << 16) |
           (acc[(m * 4 + 3) * 32 + lane] << 24);
@@ -495,6 +499,14 @@ __global__ void __launch_bounds__(kThreads, 2) dedisperse_bytes_batch_kernel(con
   const uint32_t local = s_local;
   bytes_cta<uint32_t>(sp, local % sp.grid_x, static_cast<int>(local / sp.grid_x), smem, ps);
 }
+
+}  // namespace
+}  // namespace gf
+
+#include "dedisperse_mma.cuh"
+
+namespace gf {
+namespace {
 
 // Stage-2 sum over uint32 intermediate rows (subband with 8-bit input, where
 // partial sums exceed a byte): out[dm][t] = sum_b inter[b][t + r(dm, b)].
@@ -642,6 +654,25 @@ Records build_records(const std::vector<int32_t>& delays, int ngroups, int ndm_g
   return r;
 }
 
+// Every launch of a kernel sets the same limit, whatever its own size: calls
+// from several threads would otherwise lower it under one another's launches.
+constexpr size_t kBytesMaxSmem = 224 * 1024;
+template <typename K>
+void set_max_smem(K kernel, size_t bytes) {
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+             "cudaFuncSetAttribute(dedisperse smem)");
+}
+
+// The tensor-core kernel runs where all DMs of the program make at least this
+// many of its CTAs (32768 DM-samples each); fewer leave SMs idle, and the byte
+// kernel's CTAs are a quarter of the size.  Byte kernel's automatic shape over
+// tensor-core kernel, 1100-1700 MHz:
+//   dense, 512 channels, 512 CTAs: 2.2x at DM step 0.25, 2.0x at 0.5;
+//     64 channels, 256 CTAs: 2.0x, 2.0x
+//   slices, 512 channels, 512 CTAs: 1.1-1.4x at DM steps 1-32;
+//     1024 channels: 1.06x at 224 CTAs, 0.98x at 200, 0.91x at 144-160
+constexpr uint64_t kMmaMinCtasDense = 148, kMmaMinCtasSlices = 212;
+
 struct Launch {
   int dms_per_cta = kWarps;
   int warps_per_dm = 1;
@@ -661,7 +692,7 @@ struct Launch {
 template <typename F>
 Launch choose_launch(F&& max_off_for, int dpc_fix, int cr_fix) {
   const size_t acc = static_cast<size_t>(kWarps) * kWords * 4 * 32 * 4;  // 32-bit sums
-  const size_t budget2 = 112 * 1024 - acc, budget1 = 224 * 1024 - acc;
+  const size_t budget2 = 112 * 1024 - acc, budget1 = kBytesMaxSmem - acc;
   for (size_t budget : {budget2, budget1}) {
     for (int dpc : {8, 4, 2, 1}) {
       if (dpc_fix && dpc != dpc_fix) continue;
@@ -707,9 +738,13 @@ struct BytesStage {
   Records rec;
   DeviceBlob base_dev, rec_dev, status_dev;
   int ngroups = 0, ndm_group = 0, rows_per_group = 0, total_rows = 0, blocks = 0;
+  // tensor-core path (mma.dms > 0: every launch of this stage takes it)
+  MmaShape mma;
+  int mma_blocks = 0;
+  DeviceBlob mma_base_dev, mma_rec_dev;
 
-  void build(const std::vector<int32_t>& delays, int ng, int ndg, int rpg, int tr, int device, int dpc_fix = 0,
-             int cr_fix = 0) {
+  void build(const std::vector<int32_t>& delays, int ng, int ndg, int rpg, int tr, uint64_t nout, int device,
+             int dpc_fix = 0, int cr_fix = 0) {
     ngroups = ng;
     ndm_group = ndg;
     rows_per_group = rpg;
@@ -717,11 +752,22 @@ struct BytesStage {
     launch = choose_launch([&](int dpc) { return max_off_estimate(delays, ng, ndg, rpg, tr, dpc); }, dpc_fix,
                            cr_fix);
     blocks = static_cast<int>(ceil_div(ndg, launch.dms_per_cta));
+    const uint32_t zero = 0;
+    status_dev.upload(&zero, sizeof zero, device);
+    // a pinned launch shape is a shape of the byte kernel
+    if (!dpc_fix && !cr_fix) mma = choose_mma_shape(delays, ng, ndg, rpg, tr);
+    if (mma.dms && ng * ceil_div(ndg, mma.dms) * ceil_div(nout, static_cast<uint64_t>(mma.tiles) * kMmaTile) >=
+                       (mma.steps ? kMmaMinCtasDense : kMmaMinCtasSlices)) {
+      const MmaTables t = build_mma_tables(delays, ng, ndg, rpg, tr, mma);
+      mma_blocks = t.blocks;
+      mma_base_dev.upload(t.base.data(), t.base.size() * sizeof(int32_t), device);
+      mma_rec_dev.upload(t.records.data(), t.records.size(), device);
+      return;
+    }
+    mma = MmaShape{};
     rec = build_records(delays, ng, ndg, rpg, tr, launch.dms_per_cta, launch.chunk_rows, launch.row_bytes);
     base_dev.upload(rec.base.data(), rec.base.size() * sizeof(int32_t), device);
     rec_dev.upload(rec.words.data(), rec.words.size() * sizeof(uint32_t), device);
-    const uint32_t zero = 0;
-    status_dev.upload(&zero, sizeof zero, device);
   }
 
   // Reads and clears the status word (GF_STATUS_PIPELINE: a launch gave up).
@@ -734,7 +780,9 @@ struct BytesStage {
     return v;
   }
 
-  uint64_t metadata_bytes() const { return base_dev.bytes + rec_dev.bytes; }
+  uint64_t metadata_bytes() const {
+    return base_dev.bytes + rec_dev.bytes + mma_base_dev.bytes + mma_rec_dev.bytes;
+  }
 
   // Launch for groups [g0, g0 + gcount) and, within each group, DMs
   // [dm_first, dm_first + dm_count) (dm_first a multiple of the DM block);
@@ -791,18 +839,71 @@ struct BytesStage {
     return p;
   }
 
+  // The same launch for the tensor-core kernel; dm_first is arbitrary.
+  MmaParams mma_params(const uint8_t* in, uint64_t row_stride, uint64_t group_stride, uint64_t valid, int g0,
+                       int gcount, int dm_first, int dm_count, int dm_count_last, void* out,
+                       uint64_t out_row_stride, uint64_t out_dm_rows, uint64_t out_group_rows,
+                       uint64_t nout) const {
+    check_arg(reinterpret_cast<uintptr_t>(in) % 16 == 0 && row_stride % 16 == 0 && group_stride % 16 == 0,
+              "dedispersion input must be 16-byte aligned");
+    check_arg(valid <= row_stride, "dedispersion row stride below the valid samples");
+    MmaParams p{};
+    p.in = in;
+    p.in_row_stride = row_stride;
+    p.in_group_stride = group_stride;
+    p.in_valid = valid;
+    p.rows_per_group = rows_per_group;
+    p.total_rows = total_rows - g0 * rows_per_group;
+    p.dms = mma.dms;
+    p.tiles = mma.tiles;
+    p.steps = mma.steps;
+    p.row_bytes = mma.row_bytes;
+    p.stage_bytes = mma.stage_bytes;
+    p.stages = mma.stages;
+    const int b0 = dm_first / mma.dms;
+    p.dm_skip = dm_first % mma.dms;
+    p.base_block_stride = static_cast<uint64_t>(rows_per_group);
+    p.base_group_stride = static_cast<uint64_t>(mma_blocks) * p.base_block_stride;
+    p.base = mma_base_dev.as<int32_t>() + g0 * p.base_group_stride + b0 * p.base_block_stride;
+    p.rec_block_stride = p.base_block_stride * mma_record_bytes(mma);
+    p.rec_group_stride = p.base_group_stride * mma_record_bytes(mma);
+    p.records = mma_rec_dev.as<uint8_t>() + g0 * p.rec_group_stride + b0 * p.rec_block_stride;
+    p.dm_count = dm_count;
+    p.dm_count_last = dm_count_last;
+    p.ngroups = gcount;
+    p.nblocks = static_cast<int>(ceil_div(p.dm_skip + std::max(dm_count, dm_count_last), mma.dms));
+    p.out = out;
+    p.out_row_stride = out_row_stride;
+    p.out_dm_rows = out_dm_rows;
+    p.out_group_rows = out_group_rows;
+    p.nout = nout;
+    const uint64_t ctas = ceil_div(nout, static_cast<uint64_t>(mma.tiles) * kMmaTile) *
+                          static_cast<uint64_t>(p.nblocks);
+    if (ctas >= (1ull << 31)) raise(GF_EINVAL, "dedispersion launch too large");
+    p.grid_x = static_cast<uint32_t>(ctas);
+    p.status = status_dev.as<uint32_t>();
+    return p;
+  }
+
   template <typename OutT>
   void run(const uint8_t* in, uint64_t row_stride, uint64_t group_stride, uint64_t valid, int g0,
            int gcount, int dm_first, int dm_count, int dm_count_last, void* out,
            uint64_t out_row_stride, uint64_t out_dm_rows, uint64_t out_group_rows, uint64_t nout,
            cudaStream_t stream) const {
+    if (mma.dms) {
+      const MmaParams p = mma_params(in, row_stride, group_stride, valid, g0, gcount, dm_first, dm_count,
+                                     dm_count_last, out, out_row_stride, out_dm_rows, out_group_rows, nout);
+      auto kernel = mma.steps ? dedisperse_mma_kernel<OutT, true> : dedisperse_mma_kernel<OutT, false>;
+      set_max_smem(kernel, kMmaBudget);
+      kernel<<<dim3(p.grid_x, 1u, static_cast<unsigned>(gcount)), kMmaThreads, mma.smem, stream>>>(p);
+      cuda_check(cudaGetLastError(), "dedisperse_mma_kernel launch");
+      return;
+    }
     const BytesParams p = params(in, row_stride, group_stride, valid, g0, gcount, dm_first, dm_count,
                                  dm_count_last, out, out_row_stride, out_dm_rows, out_group_rows, nout);
     dim3 grid(p.grid_x, 1u, static_cast<unsigned>(gcount));
     auto kernel = dedisperse_bytes_kernel<OutT>;
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(launch.smem)),
-               "cudaFuncSetAttribute(dedisperse smem)");
+    set_max_smem(kernel, kBytesMaxSmem);
     kernel<<<grid, kThreads, launch.smem, stream>>>(p);
     cuda_check(cudaGetLastError(), "dedisperse_bytes_kernel launch");
   }
@@ -902,7 +1003,7 @@ extern "C" int gf_dedisp_program_create(const gf_dedisp_desc* desc, gf_dedisp_pr
         for (uint64_t c = 0; c < P.nc; ++c)
           delays[dm * P.nc + c] = delay_bins(v, P.freq[d.chan_begin + c], d.ref_frequency_mhz, d.tsamp);
       }
-      P.brute.build(delays, 1, static_cast<int>(d.ndm), nc, nc, d.device_id, d.launch_dms_per_cta,
+      P.brute.build(delays, 1, static_cast<int>(d.ndm), nc, nc, P.nout, d.device_id, d.launch_dms_per_cta,
                     d.launch_chunk_rows);
     } else {
       // dedispersion.cpp:360-388 subband geometry and tables
@@ -929,7 +1030,7 @@ extern "C" int gf_dedisp_program_create(const gf_dedisp_desc* desc, gf_dedisp_pr
                 delay_bins(nominal, P.freq[d.chan_begin + c], d.ref_frequency_mhz, d.tsamp);
           }
         }
-      P.stage1.build(coarse, static_cast<int>(P.nsb), static_cast<int>(P.nnom), sbc, nc, d.device_id);
+      P.stage1.build(coarse, static_cast<int>(P.nsb), static_cast<int>(P.nnom), sbc, nc, d.nsamples, d.device_id);
       // stage 2: groups = nominal DMs, "DMs" = final DMs, rows = subbands
       P.resid.assign(P.nnom * P.npn * P.nsb, 0);
       for (uint64_t dm = 0; dm < d.ndm; ++dm) {
@@ -948,7 +1049,7 @@ extern "C" int gf_dedisp_program_create(const gf_dedisp_desc* desc, gf_dedisp_pr
       if (P.inter_u8) {
         P.inter_row_stride = round_up(P.inter_len, 16);
         P.stage2.build(P.resid, static_cast<int>(P.nnom), static_cast<int>(P.npn),
-                       static_cast<int>(P.nsb), static_cast<int>(P.nnom * P.nsb), d.device_id);
+                       static_cast<int>(P.nsb), static_cast<int>(P.nnom * P.nsb), P.nout, d.device_id);
       } else {
         P.inter_row_stride = round_up(P.inter_len, 4);
         P.resid_dev.upload(P.resid.data(), P.resid.size() * sizeof(int32_t), d.device_id);
@@ -976,8 +1077,7 @@ extern "C" int gf_dedisp_program_info(const gf_dedisp_program* P, gf_dedisp_info
       const uint64_t elem = P->inter_u8 ? 1 : 4;
       info->workspace_bytes = P->nnom * P->nsb * P->inter_row_stride * elem;
     }
-    info->metadata_bytes = P->brute.base_dev.bytes + P->brute.rec_dev.bytes + P->stage1.base_dev.bytes +
-                           P->stage1.rec_dev.bytes + P->stage2.base_dev.bytes + P->stage2.rec_dev.bytes +
+    info->metadata_bytes = P->brute.metadata_bytes() + P->stage1.metadata_bytes() + P->stage2.metadata_bytes() +
                            P->resid_dev.bytes;
   });
 }
@@ -1125,6 +1225,13 @@ struct gf_dedisp_batch {
   uint64_t blocks = 0;
   size_t smem = 0;
   DeviceBlob items_d, begin_d;
+  // items whose programs take the tensor-core kernel, by form (0: slices, 1: dense)
+  struct Mma {
+    int items = 0;
+    uint64_t blocks = 0;
+    size_t smem = 0;
+    DeviceBlob items_d, begin_d;
+  } mma[2];
 };
 
 extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_t nitems, gf_dedisp_batch** out) {
@@ -1134,7 +1241,8 @@ extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_
     check_arg(nitems > 0 && nitems < (1u << 20), "batched dedispersion takes 1 to 2^20 items");
     auto B = std::make_unique<gf_dedisp_batch>();
     std::vector<BytesParams> params;
-    std::vector<uint64_t> begin;
+    std::vector<MmaParams> mma_params[2];
+    std::vector<uint64_t> begin, mma_begin[2];
     for (uint64_t i = 0; i < nitems; ++i) {
       const gf_dedisp_batch_item& it = items[i];
       check_arg(it.program && it.dev_staged && it.dev_out, "null argument");
@@ -1147,6 +1255,18 @@ extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_
                 "DM range out of bounds");
       check_arg(it.dm_begin % 8 == 0, "dm_begin must be a multiple of 8");
       check_arg(it.out_stride >= P->nout, "out_stride must be >= nout");
+      if (P->brute.mma.dms) {
+        const int form = P->brute.mma.steps ? 1 : 0;
+        mma_params[form].push_back(P->brute.mma_params(static_cast<const uint8_t*>(it.dev_staged), P->row_stride, 0,
+                                                       d.nsamples, 0, 1, static_cast<int>(it.dm_begin),
+                                                       static_cast<int>(it.dm_count), static_cast<int>(it.dm_count),
+                                                       it.dev_out, it.out_stride, 1, 0, P->nout));
+        gf_dedisp_batch::Mma& m = B->mma[form];
+        mma_begin[form].push_back(m.blocks);
+        m.blocks += mma_params[form].back().grid_x;
+        m.smem = std::max(m.smem, P->brute.mma.smem);
+        continue;
+      }
       const BytesParams bp = P->brute.params(static_cast<const uint8_t*>(it.dev_staged), P->row_stride, 0,
                                              d.nsamples, 0, 1, static_cast<int>(it.dm_begin),
                                              static_cast<int>(it.dm_count), static_cast<int>(it.dm_count),
@@ -1156,9 +1276,16 @@ extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_
       B->smem = std::max(B->smem, P->brute.launch.smem);
       params.push_back(bp);
     }
-    check_arg(B->blocks < (1ull << 31), "batched dedispersion launch too large");
-    B->nitems = static_cast<int>(nitems);
+    check_arg(B->blocks < (1ull << 31) && B->mma[0].blocks < (1ull << 31) && B->mma[1].blocks < (1ull << 31),
+              "batched dedispersion launch too large");
+    B->nitems = static_cast<int>(params.size());
     DeviceGuard dg(B->device);
+    for (int form = 0; form < 2; ++form) {
+      gf_dedisp_batch::Mma& m = B->mma[form];
+      m.items = static_cast<int>(mma_params[form].size());
+      m.items_d.upload(mma_params[form].data(), mma_params[form].size() * sizeof(MmaParams), B->device);
+      m.begin_d.upload(mma_begin[form].data(), mma_begin[form].size() * sizeof(uint64_t), B->device);
+    }
     B->items_d.upload(params.data(), params.size() * sizeof(BytesParams), B->device);
     B->begin_d.upload(begin.data(), begin.size() * sizeof(uint64_t), B->device);
     *out = B.release();
@@ -1169,9 +1296,17 @@ extern "C" int gf_dedisp_batch_run(gf_dedisp_batch* B, void* stream) {
   return guarded([&] {
     check_arg(B != nullptr, "null argument");
     DeviceGuard dg(B->device);
-    cuda_check(cudaFuncSetAttribute(dedisperse_bytes_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(B->smem)),
-               "cudaFuncSetAttribute(dedisperse batch smem)");
+    for (int form = 0; form < 2; ++form) {
+      const gf_dedisp_batch::Mma& m = B->mma[form];
+      if (m.items == 0) continue;
+      auto kernel = form ? dedisperse_mma_batch_kernel<true> : dedisperse_mma_batch_kernel<false>;
+      set_max_smem(kernel, kMmaBudget);
+      kernel<<<static_cast<unsigned>(m.blocks), kMmaThreads, m.smem, as_stream(stream)>>>(
+          m.items_d.as<MmaParams>(), m.begin_d.as<uint64_t>(), m.items);
+      cuda_check(cudaGetLastError(), "dedisperse_mma_batch_kernel launch");
+    }
+    if (B->nitems == 0) return;
+    set_max_smem(dedisperse_bytes_batch_kernel, kBytesMaxSmem);
     dedisperse_bytes_batch_kernel<<<static_cast<unsigned>(B->blocks), kThreads, B->smem, as_stream(stream)>>>(
         B->items_d.as<BytesParams>(), B->begin_d.as<uint64_t>(), B->nitems);
     cuda_check(cudaGetLastError(), "dedisperse_bytes_batch_kernel launch");

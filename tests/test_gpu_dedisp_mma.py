@@ -1,0 +1,110 @@
+"""Dedispersion sums at the sizes where the tensor-core kernel's tiling can go
+wrong: tile edges (2048 samples, 16 DMs per CTA, 32 channels per base fetch),
+ragged DM ranges that start inside a DM block, delay spreads from none to many
+steps per DM, rows that end off a 16-byte boundary, and both stages of the
+subband path.  Sums are integers, so every comparison is exact."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def observation(nchans, nsamples, f_low=1200.0, f_high=1500.0, seed=0, levels=256):
+    rng = np.random.default_rng(seed)
+    freq = np.linspace(f_low, f_high, nchans) if nchans > 1 else np.array([f_low])
+    return freq, rng.integers(0, levels, size=(nsamples, nchans), dtype=np.uint8)
+
+
+def run(prog, data, b0, cnt):
+    staged = prog.stage(torch.from_numpy(data).cuda())
+    got = prog.run(staged, b0, cnt)[:, : prog.nout]
+    prog.check()
+    return got.cpu().numpy().view(np.uint32)
+
+
+# (channels, samples, DMs, dm_low, dm_step, first DM, DM count): enough samples
+# for the tensor-core kernel with 16, 8, 4, 2 and 1 DMs per CTA
+SHAPES = [
+    (61, 160001, 19, 0.0, 2.0, 0, 19),
+    (33, 50 * 2048 + 240, 40, 0.0, 0.1, 8, 21),
+    (257, 75 * 2048 + 301, 24, 5.0, 0.39, 8, 16),
+    (64, 55 * 2048 + 77, 33, 0.0, 7.0, 16, 17),
+    (96, 320000, 9, 0.0, 40.0, 8, 1),
+    (8, 420000, 5, 100.0, 150.0, 0, 5),
+    (40, 151 * 2048, 16, 30.0, 0.01, 0, 16),
+    (5, 4900037, 1, 0.5, 1.6, 0, 1),
+    (13, 2430011, 2, 10.0, 30.0, 0, 2),
+    (9, 1230003, 3, 10.0, 0.5, 0, 3),
+    # too few CTAs for it: the byte kernel
+    (1, 17, 1, 0.0, 1.0, 0, 1),
+    (300, 6161, 16, 30.0, 0.01, 0, 16),
+]
+
+
+@pytest.mark.parametrize("nchans,nsamples,ndm,dm_low,dm_step,b0,cnt", SHAPES)
+def test_sums_match_oracle(port, nchans, nsamples, ndm, dm_low, dm_step, b0, cnt):
+    from gaffa_b200 import core
+    freq, data = observation(nchans, nsamples, seed=nchans)
+    fref = float(freq.max()) if nchans > 1 else 1500.0
+    tsamp = 1e-3 if nchans == 1 else 256e-6
+    prog = core.DedispersionProgram(freq, nsamples, tsamp, dm_low, dm_step, ndm, ref_frequency_mhz=fref)
+    want = port.dedisperse_multi_dm(data, freq, dm_low, dm_step, ndm, fref, tsamp)
+    assert np.array_equal(run(prog, data, b0, cnt), want[b0:b0 + cnt])
+
+
+@pytest.mark.parametrize("nout_mod", [-1, 0, 1, 2047])
+def test_outputs_stay_inside_their_rows(nout_mod):
+    """Odd row ends and an unaligned output: no sample past nout is written."""
+    from gaffa_b200 import core
+    freq, data = observation(40, 6000)
+    probe = core.DedispersionProgram(freq, 6000, 256e-6, 0.0, 1.0, 16)
+    n = 6000 - probe.nout + 150 * 2048 + nout_mod
+    freq, data = observation(40, n)
+    prog = core.DedispersionProgram(freq, n, 256e-6, 0.0, 1.0, 16)
+    assert prog.nout == 150 * 2048 + nout_mod
+    staged = prog.stage(torch.from_numpy(data).cuda())
+    want = prog.run(staged)[:, : prog.nout].clone()
+    stride = prog.nout + 3
+    flat = torch.full((16 * stride + 1,), -7, dtype=torch.int32, device="cuda")
+    out = prog.run(staged, out=flat[1:], out_stride=stride)
+    prog.check()
+    assert torch.equal(out[:, : prog.nout], want)
+    assert bool((out[:, prog.nout:] == -7).all()) and int(flat[0]) == -7
+
+
+@pytest.mark.parametrize("nbits,sbc,npn,ndm", [(2, 16, 7, 25), (2, 64, 55, 60), (8, 16, 32, 40), (2, 85, 3, 11)])
+def test_subband_sums_match_oracle(port, nbits, sbc, npn, ndm):
+    from gaffa_b200 import core, synth
+    levels = 4 if nbits == 2 else 256
+    freq, data = observation(200, 30011, 300.0, 400.0, seed=npn, levels=levels)
+    raw = synth.pack_2bit(data) if nbits == 2 else data
+    prog = core.DedispersionProgram(freq, 30011, 1e-3, 0.0, 0.5, ndm, nbits=nbits, algorithm="subband",
+                                    subband_channels=sbc, ndm_per_nominal=npn)
+    want = port.dedisperse_subband(data, freq, 0.0, 0.5, ndm, float(freq.max()), 1e-3, sbc, npn)
+    assert np.array_equal(run(prog, raw, 0, ndm), want)
+    if ndm > npn:
+        assert np.array_equal(run(prog, raw, npn, ndm - npn), want[npn:])
+
+
+def test_batch_of_both_kernels_matches_single_launches():
+    from gaffa_b200 import core
+    items, want = [], []
+    for nchans, nsamples, ndm, b0, cnt in ((61, 160001, 24, 8, 13), (40, 5000, 17, 0, 17), (37, 2048 * 80, 33, 0, 33)):
+        freq, data = observation(nchans, nsamples, seed=ndm)
+        prog = core.DedispersionProgram(freq, nsamples, 256e-6, 0.0, 1.5, ndm)
+        staged = prog.stage(torch.from_numpy(data).cuda())
+        stride = (prog.nout + 3) // 4 * 4
+        want.append(prog.run(staged, b0, cnt)[:, : prog.nout].clone())
+        items.append((prog, staged, b0, cnt, torch.full((cnt * stride,), -1, dtype=torch.int32, device="cuda"), stride))
+    core.DedispersionBatch(items).run()
+    for (prog, _, _, cnt, out, stride), w in zip(items, want):
+        prog.check()
+        assert torch.equal(out.view(cnt, stride)[:, : prog.nout], w)
