@@ -584,6 +584,68 @@ __global__ void __launch_bounds__(256) stage_kernel(const uint8_t* __restrict__ 
   }
 }
 
+// 4 x 4 byte transpose: byte t of r[k] <- byte k of x[t].
+__device__ __forceinline__ void transpose4(const uint32_t (&x)[4], uint32_t (&r)[4]) {
+  const uint32_t a = __byte_perm(x[0], x[1], 0x5140), b = __byte_perm(x[2], x[3], 0x5140);
+  const uint32_t c = __byte_perm(x[0], x[1], 0x7362), d = __byte_perm(x[2], x[3], 0x7362);
+  r[0] = __byte_perm(a, b, 0x5410);
+  r[1] = __byte_perm(a, b, 0x7632);
+  r[2] = __byte_perm(c, d, 0x5410);
+  r[3] = __byte_perm(c, d, 0x7632);
+}
+
+// The same staging for 4-byte aligned rows (8-bit: nchans and chan_begin
+// multiples of 4; 2-bit: of 16): 128 samples x Chans channels per CTA, words on
+// both sides of a byte transpose in registers, so global accesses are 128-byte
+// runs (2-bit input: 64).  HBM bound: one read and one write of the data; at
+// 4096 channels the byte-wise kernel above ran at 1.3 TB/s (8-bit) and
+// 0.7 TB/s (2-bit).  A tile's word (channel c, samples 4 f ..) sits at column
+// (f + c / G) mod 32 of row c, G channels per input word, so that neither side
+// meets bank conflicts.
+template <int Bits, int Chans>
+__global__ void __launch_bounds__(256) stage_words_kernel(const uint8_t* __restrict__ in, uint64_t nsamples,
+                                                          uint64_t in_row_bytes, int chan_begin, int nchan,
+                                                          uint8_t* __restrict__ out, uint64_t out_stride,
+                                                          uint64_t t_offset) {
+  constexpr int G = 32 / Bits;           // channels per input word
+  constexpr int kRowWords = Chans / G;   // input words per sample
+  constexpr int kFours = 32;             // groups of 4 samples
+  __shared__ uint32_t tile[Chans * kFours];
+  const uint64_t tb = static_cast<uint64_t>(blockIdx.x) * (4 * kFours);
+  const int cb = blockIdx.y * Chans;
+  const uint8_t* src = in + (chan_begin + cb) / (8 / Bits);
+  for (int i = threadIdx.x; i < kRowWords * kFours; i += 256) {
+    const int w = i % kRowWords, f = i / kRowWords;
+    const uint64_t t = tb + 4 * f;
+    uint32_t x[4] = {0u, 0u, 0u, 0u};
+    if (cb + w * G < nchan) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (t + j < nsamples) x[j] = __ldcs(reinterpret_cast<const uint32_t*>(src + (t + j) * in_row_bytes) + w);
+    }
+    const int column = (f + w) % kFours;
+#pragma unroll
+    for (int j = 0; j < G / 4; ++j) {
+      uint32_t y[4], r[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = Bits == 8 ? x[q] : (x[q] >> (2 * j)) & 0x03030303u;
+      transpose4(y, r);
+      // byte k of a 2-bit word holds channels 4 k + j
+#pragma unroll
+      for (int k = 0; k < 4; ++k) tile[(w * G + (Bits == 8 ? k : 4 * k + j)) * kFours + column] = r[k];
+    }
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < Chans && cb + c < nchan; c += 8) {
+    const uint64_t t = tb + 4 * lane;
+    // the row's padding holds the rest of the last word
+    if (t < nsamples)
+      *reinterpret_cast<uint32_t*>(out + static_cast<uint64_t>(cb + c) * out_stride + t_offset + t) =
+          tile[c * kFours + (lane + c / G) % kFours];
+  }
+}
+
 // Class-sorted gather records: word 0 packs the four class counts (channels
 // of byte class 0..3), then (chunk_rows + 4) / 2 words of u16 entry pairs
 // (word offsets into the stage: row * row_bytes / 4 + delay offset / 4).
@@ -1088,6 +1150,18 @@ void launch_stage(const gf_dedisp_program& P, const uint8_t* in, uint64_t nsampl
                   uint64_t t_offset, cudaStream_t stream) {
   const auto& d = P.desc;
   const uint64_t row_bytes = d.nbits == 8 ? d.nchans : d.nchans / 4;
+  const int group = d.nbits == 8 ? 4 : 16;  // channels per word
+  if (d.nchans % group == 0 && d.chan_begin % group == 0 && P.nc % group == 0 &&
+      (reinterpret_cast<uintptr_t>(in) & 3u) == 0 && (reinterpret_cast<uintptr_t>(out) & 3u) == 0) {
+    // t_offset is a multiple of 64 and rows of 16, so words stay aligned
+    const int chans = d.nbits == 8 ? 128 : 256;
+    const dim3 grid(static_cast<unsigned>(ceil_div(nsamples, 128)), static_cast<unsigned>(ceil_div(P.nc, chans)));
+    auto kernel = d.nbits == 8 ? stage_words_kernel<8, 128> : stage_words_kernel<2, 256>;
+    kernel<<<grid, 256, 0, stream>>>(in, nsamples, row_bytes, static_cast<int>(d.chan_begin),
+                                     static_cast<int>(P.nc), out, P.row_stride, t_offset);
+    cuda_check(cudaGetLastError(), "stage_words_kernel launch");
+    return;
+  }
   dim3 grid(static_cast<unsigned>(ceil_div(nsamples, 64)), static_cast<unsigned>(ceil_div(P.nc, 64)));
   if (d.nbits == 8)
     stage_kernel<8><<<grid, 256, 0, stream>>>(in, nsamples, row_bytes, static_cast<int>(d.chan_begin),

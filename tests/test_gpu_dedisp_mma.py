@@ -108,3 +108,19 @@ def test_batch_of_both_kernels_matches_single_launches():
     for (prog, _, _, cnt, out, stride), w in zip(items, want):
         prog.check()
         assert torch.equal(out.view(cnt, stride)[:, : prog.nout], w)
+
+
+@pytest.mark.parametrize("nbits,nchans,nsamples,begin,end", [
+    (8, 132, 1000, 0, 132), (8, 132, 129, 4, 128), (8, 132, 127, 3, 130), (8, 61, 300, 0, 61),
+    (2, 272, 515, 0, 272), (2, 272, 128, 16, 256), (2, 272, 131, 4, 271), (2, 20, 64, 0, 20)])
+def test_staging_is_the_transpose(nbits, nchans, nsamples, begin, end):
+    from gaffa_b200 import core, synth
+    freq, data = observation(nchans, nsamples, seed=nsamples, levels=4 if nbits == 2 else 256)
+    raw = synth.pack_2bit(data) if nbits == 2 else data
+    prog = core.DedispersionProgram(freq, nsamples, 1e-3, 0.0, 0.01, 1, chan_begin=begin, chan_end=end, nbits=nbits,
+                                    ref_frequency_mhz=1500.0)
+    want = torch.from_numpy(np.ascontiguousarray(data[:, begin:end].T)).cuda()
+    stride = int(prog.info.staged_row_stride)
+    for src in (torch.from_numpy(raw).cuda(), raw):   # device input, and host input through the bounce buffer
+        got = prog.stage(src).view(end - begin, stride)[:, :nsamples]
+        assert torch.equal(got, want)
