@@ -15,18 +15,16 @@
 // Execution.  The recursion tree is processed by depth: every node at depth d
 // splits [a, a+n) into head [a, a+n/2) and tail [a+n/2, a+n); a node of one row
 // is the input row itself.  A task whose rows fit a CTA's shared memory runs in
-// one CTA (all levels on chip, root rows fed straight into detection).  Larger
-// tasks run on a thread-block cluster: each CTA transforms subtrees of at most
-// max_rows rows on chip and writes them to the cluster's global scratch; then
-// column passes of up to three levels each climb to the root.  A column block
-// computes a run of rows of one node from the rows three levels down that it
-// depends on (the schedules are built on the host, once per program); blocks
-// of a pass are split across the cluster's CTAs, and a hardware cluster
-// barrier separates passes.  The root pass is fused with detection.  Kernels
-// are instantiated per NB = ceil(bins / 32) so every row loop is unrolled.
+// one CTA (all levels on chip, root rows fed straight into detection).  A larger
+// task is transformed in subtrees of at most max_rows rows, written to the
+// CTA's global scratch; column passes of up to three levels each climb to the
+// root.  A column block computes a run of rows of one node from the rows three
+// levels down that it depends on (the schedules are built on the host, once per
+// program).  The first pass takes each of its nodes as soon as the node's
+// subtrees are done, so it reads their rows from L2; the root pass is fused
+// with detection.  Kernels are instantiated per NB = ceil(bins / 32) so every
+// row loop is unrolled.
 #include "common.cuh"
-
-#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cmath>
@@ -35,8 +33,6 @@
 #include <memory>
 #include <tuple>
 #include <vector>
-
-namespace cg = cooperative_groups;
 
 namespace gf {
 namespace {
@@ -48,15 +44,10 @@ namespace {
 // prepare pass.
 constexpr int kThreads = 1024;
 constexpr int kSmallThreads = 512;
+constexpr size_t kSmallSmem = 110 * 1024, kLargeSmem = 222 * 1024;
 constexpr int kPrepareThreads = 512;
 constexpr int kMaxBins = 512;
 constexpr int kMaxWidths = 64;
-// Largest thread-block cluster for one (series, task).  One CTA per item:
-// on the survey plan at 16 and 256 series, clusters of up to 8 CTAs (sized
-// by rows) ran 11-15 % slower than independent CTAs, which need no cluster
-// barriers and keep every SM busy with its own item (16-CTA clusters were
-// slower still).
-constexpr int kClusterSize = 1;
 constexpr int kPrepareChunk = 16384;
 
 struct TaskDev {
@@ -69,6 +60,7 @@ struct TaskDev {
   uint32_t max_width;
   uint32_t pass_begin;    // column passes (split_depth > 0)
   uint32_t npasses;
+  uint32_t first_depth;   // depth of the first pass's nodes
   uint32_t member;        // observation of a batched program (0 otherwise)
 };
 
@@ -232,17 +224,69 @@ __global__ void __launch_bounds__(kPrepareThreads) prepare_kernel(const __grid_c
 // A level of the tree is a list of rows, each produced by one MetaEntry:
 //   MERGE  out = prev[a] + roll_left(prev[b], roll mod bins)   (ffa.cpp:110-171)
 //   CARRY  out = prev[a]              (a one-row node carried up unchanged)
-// Rows of a level live in one of two shared-memory buffers (pitch = bins|1);
-// levels alternate buffers, so each level costs one __syncthreads.  Every
-// loop over the bins of a row is unrolled for NB = ceil(bins / 32) (the
-// kernels are instantiated per NB), so a merged element costs two shared
-// loads, one add and one shared store.
+// Levels are evaluated two at a time: a pass of QuadOps reads the rows two
+// levels down and writes groups of up to four consecutive rows, the level
+// between kept in registers.  Neighbouring rows of a node share their head
+// and tail rows (the shift of row s is split between the children as s/2 each,
+// rounded), so a group of four needs two head rows, each once, and two or three
+// tail rows, at one or two neighbouring phases each:
+//   R  outputs h0 + w0(k), h0 + w0(k+1), h1 + w1(k), h1 + w1(k+1)
+//   F  outputs h0 + w0(k), h0 + w1(k),   h1 + w1(k+1), h1 + w2(k)
+// with h_i = a_i + roll(b_i) and w_i = roll(c_i + roll(d_i)), every sum in the
+// reference's order.  RS and FS are the same with the children's own rows
+// shared (a1 = a0, b1 = b0 one phase on; likewise c, d in RS); rows that fit no
+// group are pairs (two rows of one head and tail) or single rows.  Bound:
+// shared-memory accesses -- 16 per 8 merged elements in R and F, 14 in RS and
+// FS, 8 per 4 in pairs, against 24 per 8 one level at a time -- and the warps
+// in flight that hide their latency: 1024 threads of 64 registers beat 512 of
+// 128 with twice the loads ahead (43.7 against 49.1 ms, 32 series of 2^22
+// samples on the survey plan).  Rows hold three wrapped samples past their end
+// so that neighbouring phases need no index of their own.  A task of an odd number of levels takes
+// one level by itself (MetaEntries).
+// Rows of a pass live in one of two shared-memory buffers (pitch =
+// (bins + 3) | 1); passes alternate buffers, so each costs one __syncthreads.
+// Every loop over the bins of a row is unrolled for NB = ceil(bins / 32) (the
+// kernels are instantiated per NB).
 
 enum : uint16_t { kMerge = 0, kCarry = 1 };
 
 struct __align__(8) MetaEntry {
   uint16_t op, a, b, roll;
 };
+
+enum : uint16_t { kOpR = 0, kOpRS, kOpF, kOpFS, kOpPair, kOpOne };
+constexpr uint32_t kHalo = 3;   // wrapped samples kept past the end of a row
+
+// Group of output rows row, row + 1, ...; rolls are phases relative to the
+// output (rd: of d itself, the tail's roll included).
+struct __align__(16) QuadOp {
+  uint16_t type, row;
+  uint16_t a[2], b[2], rb[2];
+  uint16_t c[3], d[3], rc[3], rd[3];
+  uint16_t flags;               // kOpOne: 1 = b present, 2 = c present, 4 = d present
+  uint16_t pad[3];
+};
+static_assert(sizeof(QuadOp) == 48, "QuadOp is three 16-byte words");
+
+// A pass: bit 15 = two levels (QuadOps) or one (MetaEntries); low bits the count.
+constexpr uint16_t kPassTwo = 0x8000;
+constexpr int kMaxPasses = 10;
+__host__ __device__ __forceinline__ uint32_t pass_bytes(uint16_t pass) {
+  const uint32_t n = pass & 0x7fffu;
+  return pass & kPassTwo ? n * static_cast<uint32_t>(sizeof(QuadOp))
+                         : (n * static_cast<uint32_t>(sizeof(MetaEntry)) + 15u) & ~15u;
+}
+
+// Schedule of a whole subtree of n rows: passes from the leaves to the root.
+// The head also leads the staged entries.
+struct __align__(16) SubHead {
+  uint32_t offset16;            // first 16-byte word of the passes' entries
+  uint16_t size16;
+  uint16_t npasses;
+  uint16_t pass[kMaxPasses];
+  uint16_t pad[2];
+};
+static_assert(sizeof(SubHead) == 32, "SubHead is two 16-byte words");
 
 struct Node {
   uint32_t a, n, depth;
@@ -287,24 +331,21 @@ __device__ __forceinline__ uint32_t scaled_shift(float scale, uint32_t s) {
   return static_cast<uint32_t>(__fadd_rn(__fmul_rn(scale, static_cast<float>(s)), 0.5f));
 }
 
-__host__ __device__ __forceinline__ uint32_t tree_depth(uint32_t n) {
-  uint32_t d = 0;
-  while (n > 1) { n = (n + 1) >> 1; ++d; }
-  return d;
-}
-
 // A column block of a pass (built on the host): rows [s0, s1) of one node X
 // at depth dx, evaluated from the rows of depth dx + levels that they depend
-// on.  Level k (0 = X) holds count[k] rows; the bottom level is loaded from
-// the pass's source scratch as up to 8 runs of consecutive task rows.
+// on.  The bottom level is loaded from the pass's source scratch as up to 8
+// runs of consecutive task rows.
 struct ColBlock {
-  uint32_t meta;          // first merge entry: levels-1, ..., 0 back to back
+  uint32_t meta16;        // first 16-byte word of the passes' entries, bottom pass first
   uint32_t out_row;       // final pass: shift of the first root row; else task row of the first output row
-  uint16_t count[4];      // rows at relative level 0 .. levels
+  uint16_t rows;          // output rows
+  uint16_t nbottom;       // bottom rows
+  uint16_t size16;        // entries in 16-byte words
+  uint16_t pass[3];
   uint16_t run_off[8];    // bottom level: buffer row where each run starts
   uint16_t run_row[8];    // bottom level: task row where each run starts
-  uint8_t levels, final_pass, nruns, reserved;
-  uint32_t pad[3];
+  uint8_t npasses, final_pass, nruns, reserved;
+  uint32_t pad[2];
 };
 static_assert(sizeof(ColBlock) == 64, "ColBlock is 16 words");
 
@@ -312,82 +353,275 @@ struct PassDev {
   uint32_t block_begin, nblocks;
 };
 
-// Search-path device functions take the CTA size T (512 or 1024 threads).
+// Search-path device functions take the CTA size T (512 or 1024 threads).  The
+// ones that merge or detect are inlined: as calls, their register saves and
+// the caller's cost 2 % on the survey plan and 17 % on 48-64 bins.
 
 // Dynamic shared memory of the search kernel: two ColBlock headers, the
 // staged schedule, then two row buffers.
 extern __shared__ __align__(16) float g_smem[];
 
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// One level: out row q (q < nrows) from `prev` by meta[q].  A warp per row,
-// lane j handles bins j, j+32, ...; only the last iteration can be partial.
-// The tail row is read at k = (j + roll) mod bins, computed branch-free as
-// min(k, k - bins) in unsigned arithmetic (k < 2 bins).
-template <int NB, int T>
-__device__ __forceinline__ void merge_level(const MetaEntry* meta, uint32_t nrows, const float* prev, float* out,
-                                            uint32_t pitch, uint32_t bins) {
+// A row read `roll` phases on, in g_smem indexes: lane j's sample of bins
+// j + 32 i is at(i), its neighbours after it (kHalo wrapped samples follow a
+// row).  The wrap past the row's end is one select per 32 bins.
+struct RolledRow {
+  uint32_t p, wrapped;
+  int32_t w;
+  __device__ __forceinline__ RolledRow(uint32_t row, uint32_t roll, uint32_t bins, uint32_t lane) {
+    if (roll >= bins) roll %= bins;
+    p = row + lane + roll;
+    wrapped = p - bins;
+    w = static_cast<int32_t>(lane + roll) - static_cast<int32_t>(bins);
+  }
+  __device__ __forceinline__ const float* at(int i) const {
+    // opaque, or the selects of a whole row are formed ahead and spill
+    int32_t v = w;
+    asm volatile("" : "+r"(v));
+    return g_smem + ((v + 32 * i >= 0 ? wrapped : p) + 32u * static_cast<uint32_t>(i));
+  }
+};
+
+// Output rows of a group: row j is written when lo <= row + j < hi, at row
+// row + j - lo of the output buffer; the first lanes write the wrapped samples.
+template <bool Clip>
+struct OutRows {
+  uint32_t first;         // g_smem index of the lane's first sample of row `row`
+  uint32_t pitch, bins, lane;
+  int32_t lo, hi;         // rows of the group to write (Clip)
+  __device__ __forceinline__ void put(int j, int i, float v) const {
+    if (Clip && (j < lo || j >= hi)) return;
+    float* o = g_smem + (first + static_cast<uint32_t>(j) * pitch + 32u * static_cast<uint32_t>(i));
+    *o = v;
+    if (i == 0 && lane < kHalo) {
+      o[bins] = v;
+      if (bins == 2 && lane == 0) o[4] = v;
+    }
+  }
+};
+
+template <int NB, bool Shared, bool Clip>
+__device__ __forceinline__ void quad_r(const QuadOp& m, uint32_t prev, uint32_t pitch, const OutRows<Clip>& out,
+                                       bool last_ok) {
+  const uint32_t lane = out.lane, bins = out.bins;
+  const float* a0 = g_smem + prev + m.a[0] * pitch + lane;
+  const float* a1 = g_smem + prev + m.a[1] * pitch + lane;
+  const RolledRow b0(prev + m.b[0] * pitch, m.rb[0], bins, lane), c0(prev + m.c[0] * pitch, m.rc[0], bins, lane),
+      d0(prev + m.d[0] * pitch, m.rd[0], bins, lane);
+  if (Shared) {
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (i < NB - 1 || last_ok) {
+        const float a = a0[32 * i];
+        const float *b = b0.at(i), *c = c0.at(i), *d = d0.at(i);
+        const float h0 = __fadd_rn(a, b[0]), h1 = __fadd_rn(a, b[1]);
+        const float c1 = c[1];
+        out.put(0, i, __fadd_rn(h0, __fadd_rn(c[0], d[0])));
+        out.put(1, i, __fadd_rn(h0, __fadd_rn(c1, d[1])));
+        out.put(2, i, __fadd_rn(h1, __fadd_rn(c1, d[2])));
+        out.put(3, i, __fadd_rn(h1, __fadd_rn(c[2], d[3])));
+      }
+  } else {
+    const RolledRow b1(prev + m.b[1] * pitch, m.rb[1], bins, lane), c1(prev + m.c[1] * pitch, m.rc[1], bins, lane),
+        d1(prev + m.d[1] * pitch, m.rd[1], bins, lane);
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (i < NB - 1 || last_ok) {
+        const float h0 = __fadd_rn(a0[32 * i], *b0.at(i)), h1 = __fadd_rn(a1[32 * i], *b1.at(i));
+        const float *c = c0.at(i), *d = d0.at(i), *e = c1.at(i), *f = d1.at(i);
+        out.put(0, i, __fadd_rn(h0, __fadd_rn(c[0], d[0])));
+        out.put(1, i, __fadd_rn(h0, __fadd_rn(c[1], d[1])));
+        out.put(2, i, __fadd_rn(h1, __fadd_rn(e[0], f[0])));
+        out.put(3, i, __fadd_rn(h1, __fadd_rn(e[1], f[1])));
+      }
+  }
+}
+
+template <int NB, bool Shared, bool Clip>
+__device__ __forceinline__ void quad_f(const QuadOp& m, uint32_t prev, uint32_t pitch, const OutRows<Clip>& out,
+                                       bool last_ok) {
+  const uint32_t lane = out.lane, bins = out.bins;
+  const float* a0 = g_smem + prev + m.a[0] * pitch + lane;
+  const float* a1 = g_smem + prev + m.a[1] * pitch + lane;
+  const RolledRow b0(prev + m.b[0] * pitch, m.rb[0], bins, lane), b1(prev + m.b[1] * pitch, m.rb[1], bins, lane);
+  const RolledRow c0(prev + m.c[0] * pitch, m.rc[0], bins, lane), d0(prev + m.d[0] * pitch, m.rd[0], bins, lane);
+  const RolledRow c1(prev + m.c[1] * pitch, m.rc[1], bins, lane), d1(prev + m.d[1] * pitch, m.rd[1], bins, lane);
+  const RolledRow c2(prev + m.c[2] * pitch, m.rc[2], bins, lane), d2(prev + m.d[2] * pitch, m.rd[2], bins, lane);
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    if (i < NB - 1 || last_ok) {
+      float h0, h1;
+      if (Shared) {
+        const float a = a0[32 * i];
+        const float* b = b0.at(i);
+        h0 = __fadd_rn(a, b[0]);
+        h1 = __fadd_rn(a, b[1]);
+      } else {
+        h0 = __fadd_rn(a0[32 * i], *b0.at(i));
+        h1 = __fadd_rn(a1[32 * i], *b1.at(i));
+      }
+      const float *c = c1.at(i), *d = d1.at(i);
+      out.put(0, i, __fadd_rn(h0, __fadd_rn(*c0.at(i), *d0.at(i))));
+      out.put(1, i, __fadd_rn(h0, __fadd_rn(c[0], d[0])));
+      out.put(2, i, __fadd_rn(h1, __fadd_rn(c[1], d[1])));
+      out.put(3, i, __fadd_rn(h1, __fadd_rn(*c2.at(i), *d2.at(i))));
+    }
+}
+
+// Two rows of one head and one tail row (Pair), or one row, any of whose four
+// inputs may be missing (rows carried up unchanged).
+template <int NB, bool Pair, bool Clip>
+__device__ __forceinline__ void quad_rest(const QuadOp& m, uint32_t prev, uint32_t pitch, const OutRows<Clip>& out,
+                                          bool last_ok) {
+  const uint32_t lane = out.lane, bins = out.bins;
+  const float* a0 = g_smem + prev + m.a[0] * pitch + lane;
+  const RolledRow b0(prev + m.b[0] * pitch, m.rb[0], bins, lane), c0(prev + m.c[0] * pitch, m.rc[0], bins, lane),
+      d0(prev + m.d[0] * pitch, m.rd[0], bins, lane);
+  const bool has_b = Pair || (m.flags & 1), has_c = Pair || (m.flags & 2), has_d = Pair || (m.flags & 4);
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    if (i < NB - 1 || last_ok) {
+      float h = a0[32 * i];
+      if (has_b) h = __fadd_rn(h, *b0.at(i));
+      if (Pair) {
+        const float *c = c0.at(i), *d = d0.at(i);
+        out.put(0, i, __fadd_rn(h, __fadd_rn(c[0], d[0])));
+        out.put(1, i, __fadd_rn(h, __fadd_rn(c[1], d[1])));
+      } else {
+        if (has_c) {
+          float w = *c0.at(i);
+          if (has_d) w = __fadd_rn(w, *d0.at(i));
+          h = __fadd_rn(h, w);
+        }
+        out.put(0, i, h);
+      }
+    }
+}
+
+__device__ __forceinline__ uint32_t op_rows(uint16_t type) { return type == kOpPair ? 2u : type == kOpOne ? 1u : 4u; }
+
+// Two levels: a warp per group, lane j handles bins j, j + 32, ...  Clip: rows
+// [lo, hi) only, written from row 0 of the output buffer.
+template <int NB, int T, bool Clip>
+__device__ __forceinline__ void merge_two(const QuadOp* ops, uint32_t nops, uint32_t prev, uint32_t out_buf,
+                                          uint32_t pitch, uint32_t bins, uint32_t lo, uint32_t hi) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool last_ok = lane + 32u * (NB - 1) < bins;
-  for (uint32_t q = warp; q < nrows; q += T / 32) {
-    const MetaEntry m = meta[q];
-    float* o = out + q * pitch + lane;
-    const float* h = prev + m.a * pitch + lane;
-    if (m.op == kMerge) {
-      uint32_t r = m.roll;
-      if (r >= bins) r %= bins;
-      const uint32_t k0 = lane + r;       // < 2 bins
-      const uint32_t k1 = k0 - bins;      // wraps when k0 < bins
-      const float* t = prev + m.b * pitch;
-#pragma unroll
-      for (int i = 0; i < NB; ++i) {
-        if (i < NB - 1 || last_ok) {
-          const uint32_t k = umin32(k0 + 32u * i, k1 + 32u * i);
-          o[32 * i] = __fadd_rn(h[32 * i], t[k]);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < NB; ++i)
-        if (i < NB - 1 || last_ok) o[32 * i] = h[32 * i];
+  for (uint32_t q = warp; q < nops; q += T / 32) {
+    const QuadOp& m = ops[q];
+    const uint16_t type = m.type;
+    const uint32_t row = m.row;
+    OutRows<Clip> out;
+    out.first = out_buf + (Clip ? row - lo : row) * pitch + lane;
+    out.pitch = pitch;
+    out.bins = bins;
+    out.lane = lane;
+    if (Clip) {
+      out.lo = static_cast<int32_t>(lo) - static_cast<int32_t>(row);
+      out.hi = static_cast<int32_t>(hi) - static_cast<int32_t>(row);
+      if (out.hi <= 0 || out.lo >= static_cast<int32_t>(op_rows(type))) continue;
+    }
+    switch (type) {
+      case kOpR: quad_r<NB, false, Clip>(m, prev, pitch, out, last_ok); break;
+      case kOpRS: quad_r<NB, true, Clip>(m, prev, pitch, out, last_ok); break;
+      case kOpF: quad_f<NB, false, Clip>(m, prev, pitch, out, last_ok); break;
+      case kOpFS: quad_f<NB, true, Clip>(m, prev, pitch, out, last_ok); break;
+      case kOpPair: quad_rest<NB, true, Clip>(m, prev, pitch, out, last_ok); break;
+      default: quad_rest<NB, false, Clip>(m, prev, pitch, out, last_ok); break;
     }
   }
 }
 
-// rows [0, n) of read-only global `src` (row length bins) into smem, async
+// One level: rows [lo, hi) of meta into rows 0, 1, ... of the output buffer.
 template <int NB, int T>
-__device__ __forceinline__ void load_rows_async(const float* src, uint32_t n, uint32_t bins, float* out,
-                                                uint32_t pitch) {
+__device__ __forceinline__ void merge_one(const MetaEntry* meta, uint32_t prev, uint32_t out_buf, uint32_t pitch,
+                                          uint32_t bins, uint32_t lo, uint32_t hi) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool last_ok = lane + 32u * (NB - 1) < bins;
-  for (uint32_t q = warp; q < n; q += T / 32) {
-    const float* g = src + static_cast<uint64_t>(q) * bins + lane;
-    float* o = out + q * pitch + lane;
+  for (uint32_t q = lo + warp; q < hi; q += T / 32) {
+    const MetaEntry m = meta[q];
+    OutRows<false> out;
+    out.first = out_buf + (q - lo) * pitch + lane;
+    out.pitch = pitch;
+    out.bins = bins;
+    out.lane = lane;
+    const float* h = g_smem + prev + m.a * pitch + lane;
+    if (m.op == kMerge) {
+      const RolledRow t(prev + m.b * pitch, m.roll, bins, lane);
 #pragma unroll
-    for (int i = 0; i < NB; ++i)
-      if (i < NB - 1 || last_ok) cp_async4(o + 32 * i, g + 32 * i);
+      for (int i = 0; i < NB; ++i)
+        if (i < NB - 1 || last_ok) out.put(0, i, __fadd_rn(h[32 * i], *t.at(i)));
+    } else {
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (i < NB - 1 || last_ok) out.put(0, i, h[32 * i]);
+    }
   }
 }
 
+// A whole pass (the root pass of an on-chip task goes by merge_rows instead).
 template <int NB, int T>
-__device__ __forceinline__ void store_rows(const float* in, uint32_t pitch, uint32_t n, uint32_t bins, float* dst) {
+__device__ __forceinline__ void run_pass(uint16_t pass, const char* meta, uint32_t prev, uint32_t out_buf,
+                                         uint32_t pitch, uint32_t bins) {
+  const uint32_t n = pass & 0x7fffu;
+  if (pass & kPassTwo)
+    merge_two<NB, T, false>(reinterpret_cast<const QuadOp*>(meta), n, prev, out_buf, pitch, bins, 0u, 0u);
+  else
+    merge_one<NB, T>(reinterpret_cast<const MetaEntry*>(meta), prev, out_buf, pitch, bins, 0u, n);
+}
+
+// Rows [lo, hi) of a pass.
+template <int NB, int T>
+__device__ __forceinline__ void merge_rows(uint16_t pass, const char* meta, uint32_t prev, uint32_t out_buf,
+                                           uint32_t pitch, uint32_t bins, uint32_t lo, uint32_t hi) {
+  if (pass & kPassTwo)
+    merge_two<NB, T, true>(reinterpret_cast<const QuadOp*>(meta), pass & 0x7fffu, prev, out_buf, pitch, bins, lo, hi);
+  else
+    merge_one<NB, T>(reinterpret_cast<const MetaEntry*>(meta), prev, out_buf, pitch, bins, lo, hi);
+}
+
+template <int NB, int I = 0>
+__device__ __forceinline__ void copy_bins_async(uint32_t to, const float* from, bool last_ok) {
+  if constexpr (I < NB) {
+    if (I < NB - 1 || last_ok)
+      asm volatile("cp.async.ca.shared.global [%0+%2], [%1+%2], 4;\n" ::"r"(to), "l"(from), "n"(128 * I) : "memory");
+    copy_bins_async<NB, I + 1>(to, from, last_ok);
+  }
+}
+
+// One row of length `bins` from global memory, wrapped samples included, async.
+template <int NB>
+__device__ __forceinline__ void load_row_async(const float* src, uint32_t bins, float* row, uint32_t lane,
+                                               bool last_ok) {
+  const float* g = src + lane;
+  const uint32_t o = static_cast<uint32_t>(__cvta_generic_to_shared(row + lane));
+  copy_bins_async<NB>(o, g, last_ok);
+  if (lane < kHalo)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(o + 4 * bins), "l"(lane < bins ? g : g - bins));
+}
+
+// rows [0, n) of read-only global `src` (row length bins) into smem, async
+template <int NB, int T>
+__device__ __forceinline__ void load_rows_async(const float* src, uint32_t n, uint32_t bins, uint32_t out,
+                                                uint32_t pitch) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool last_ok = lane + 32u * (NB - 1) < bins;
+  for (uint32_t q = warp; q < n; q += T / 32)
+    load_row_async<NB>(src + static_cast<uint64_t>(q) * bins, bins, g_smem + out + q * pitch, lane, last_ok);
+}
+
+template <int NB, int T>
+__device__ __forceinline__ void store_rows(uint32_t in, uint32_t pitch, uint32_t n, uint32_t bins, float* dst) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool last_ok = lane + 32u * (NB - 1) < bins;
   for (uint32_t q = warp; q < n; q += T / 32) {
     float* g = dst + static_cast<uint64_t>(q) * bins + lane;
-    const float* s = in + q * pitch + lane;
+    const float* s = g_smem + in + q * pitch + lane;
 #pragma unroll
     for (int i = 0; i < NB; ++i)
       if (i < NB - 1 || last_ok) __stcg(g + 32 * i, s[32 * i]);
@@ -399,7 +633,7 @@ __device__ __forceinline__ void store_rows(const float* in, uint32_t pitch, uint
 // ---------------------------------------------------------------------------
 
 struct DetectArgs {
-  const TrialDev* trials;
+  const TrialDev* trials;    // shared memory
   uint32_t ntrials, max_width, bins;
   float inv_stdnoise, threshold;
   uint32_t series, task;
@@ -417,6 +651,21 @@ __device__ __forceinline__ float key_float(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// {x0 - y0, x1 - y1}, each rounded to nearest
+__device__ __forceinline__ float2 sub2(float x0, float x1, float y0, float y1) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, d;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "sub.rn.f32x2 d, x, y;\n\tmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(x0), "f"(x1), "f"(y0), "f"(y1));
+  return d;
+}
+
 // rows[i] (pitch `pitch`) hold root rows shift0 + i, i < count.  Prefix sums
 // are sequential per row (one thread per row, ffa_detection.cpp:126-139).
 // Then a warp per row: lane j holds c[j + 32i] and, for every width, takes
@@ -425,13 +674,13 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 // threshold is the first phase attaining the maximum looked up (the
 // reference's strict '>' scan keeps the first maximum), and a peak appended.
 template <int NB, int T>
-__device__ void detect_rows(const float* rows, uint32_t pitch, uint32_t count, uint32_t shift0, float* cp,
+__device__ __forceinline__ void detect_rows(const float* rows, uint32_t pitch, uint32_t count, uint32_t shift0, float* cp,
                             uint32_t cp_pitch, const DetectArgs& a) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t bins = a.bins;
-  if (threadIdx.x < count) {
-    const float* prof = rows + threadIdx.x * pitch;
-    float* c = cp + threadIdx.x * cp_pitch;
+  for (uint32_t row = threadIdx.x; row < count; row += T) {
+    const float* prof = rows + row * pitch;
+    float* c = cp + row * cp_pitch;
     float acc = 0.0f;
     c[0] = 0.0f;
     // loads of the next 8 samples overlap the current 8-add chain
@@ -470,10 +719,15 @@ __device__ void detect_rows(const float* rows, uint32_t pitch, uint32_t count, u
     for (uint32_t k = 0; k < a.ntrials; ++k) {
       const TrialDev tr = a.trials[k];
       const float* cw = c + tr.width;
+      // two phases per packed subtraction and per three-input maximum
       float best = -INFINITY;
 #pragma unroll
-      for (int i = 0; i < NB; ++i)
-        if (i < NB - 1 || last_ok) best = fmaxf(best, __fsub_rn(cw[32 * i], base[i]));
+      for (int i = 0; i + 1 < NB - 1; i += 2) {
+        const float2 d = sub2(cw[32 * i], cw[32 * i + 32], base[i], base[i + 1]);
+        best = max3(best, d.x, d.y);
+      }
+      if (NB % 2 == 0) best = fmaxf(best, __fsub_rn(cw[32 * (NB - 2)], base[NB - 2 < 0 ? 0 : NB - 2]));
+      if (last_ok) best = fmaxf(best, __fsub_rn(cw[32 * (NB - 1)], base[NB - 1]));
       // S/N is monotone in the boxcar sum, so the row passes the threshold
       // exactly when some lane's own maximum does
       const float lane_snr = __fmul_rn(
@@ -516,9 +770,9 @@ struct SearchParams {
   uint64_t prep_stride;
   const TaskDev* tasks;
   const TrialDev* trials;
-  const MetaEntry* sub_meta;    // subtree schedules by size
-  const uint32_t* sub_offset;   // [max_rows + 1]
-  const MetaEntry* col_meta;    // column-block merge entries
+  const uint4* sub_meta;        // subtree schedules
+  const SubHead* sub_head;      // [max_rows + 1] by size
+  const uint4* col_meta;        // column-block schedules
   const ColBlock* blocks;       // column blocks, pass by pass
   const PassDev* passes;
   const uint32_t* item_tasks;   // task indices of this launch's class
@@ -532,17 +786,18 @@ struct SearchParams {
   gf_peak_record* peaks;
   uint64_t capacity;
   unsigned long long* counters;
-  float* scratch;               // per cluster: 2 * scratch_elems floats
-  uint64_t scratch_elems;
+  float* scratch;               // per CTA: scratch_elems0 + scratch_elems1 floats
+  uint64_t scratch_elems0, scratch_elems1;
   uint32_t pitch;               // shared-memory row pitch (max bins | 1)
   uint32_t max_rows;            // rows per shared-memory buffer
   uint32_t front;               // floats before the first row buffer
+  uint32_t block_rows;          // output rows of a column block (passes but the last)
 };
 
-__device__ __forceinline__ DetectArgs make_detect(const SearchParams& p, const TaskDev& t, uint32_t series,
-                                                  uint32_t task) {
+__device__ __forceinline__ DetectArgs make_detect(const SearchParams& p, const TaskDev& t, const TrialDev* trials,
+                                                  uint32_t series, uint32_t task) {
   DetectArgs da;
-  da.trials = p.trials + t.trial_offset;
+  da.trials = trials;
   da.ntrials = t.ntrials;
   da.max_width = t.max_width;
   da.bins = t.bins;
@@ -556,63 +811,84 @@ __device__ __forceinline__ DetectArgs make_detect(const SearchParams& p, const T
   return da;
 }
 
-// Evaluates a whole subtree of n <= max_rows rows (pointer `src` = its first
-// input row) from its input rows up to relative level `stop` (0: the
-// subtree root).  The subtree's schedule (depth x n entries, level depth-1
-// first) is left in cmeta.  Returns the buffer holding level `stop`.
-template <int NB, int T>
-__device__ float* eval_subtree(const SearchParams& p, const float* src, uint32_t n, uint32_t bins, uint32_t stop,
-                               float* buf0, float* buf1, MetaEntry* cmeta) {
-  const uint32_t pitch = p.pitch;
-  const uint32_t md = tree_depth(n);
-  const MetaEntry* table = p.sub_meta + p.sub_offset[n];
-  for (uint32_t e = threadIdx.x; e < md * n; e += T) cp_async8(cmeta + e, table + e);
-  load_rows_async<NB, T>(src, n, bins, (md & 1) ? buf1 : buf0, pitch);
-  cp_async_wait_all();
-  __syncthreads();
-  for (int l = static_cast<int>(md) - 1; l >= static_cast<int>(stop); --l) {
-    merge_level<NB, T>(cmeta + (md - 1 - l) * n, n, ((l + 1) & 1) ? buf1 : buf0, (l & 1) ? buf1 : buf0, pitch, bins);
-    __syncthreads();
-  }
-  return (stop & 1) ? buf1 : buf0;
+// Brings [p, p + n) floats towards L2 (whole 16-byte words inside the range):
+// 43.1 -> 42.6 ms on the survey plan.
+__device__ __forceinline__ void prefetch_l2(const float* p, uint64_t n) {
+  const uint64_t begin = (reinterpret_cast<uint64_t>(p) + 15) & ~15ull;
+  const uint64_t end = reinterpret_cast<uint64_t>(p + n) & ~15ull;
+  if (begin < end)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(begin), "r"(static_cast<uint32_t>(end - begin)));
 }
 
-// Column block `hb`: stages its merge entries, loads its bottom rows from
-// `src` (scratch written by the cluster's CTAs in the previous phase),
-// evaluates its levels.  The output rows (hb.count[0]) end in buf0.
+// Stages `size16` 16-byte words of a schedule, async.
+template <int T>
+__device__ __forceinline__ void stage_schedule(char* dst, const uint4* src, uint32_t size16) {
+  for (uint32_t e = threadIdx.x; e < size16; e += T) cp_async16(dst + 16 * e, src + e);
+}
+
+// Evaluates a subtree of n <= max_rows rows (pointer `src` = its first input
+// row) up to its last pass, or up to the pass before it when `root` (then
+// *meta is that pass's entries).  Returns the buffer that holds the result.
 template <int NB, int T>
-__device__ void eval_block(const SearchParams& p, const ColBlock& hb, const float* src, uint32_t bins, float* buf0,
-                           float* buf1, MetaEntry* cmeta) {
+__device__ __forceinline__ uint32_t eval_subtree(const SearchParams& p, const float* src, uint32_t n, uint32_t bins, bool root,
+                                 uint32_t buf0, uint32_t buf1, char* smeta, const char** meta) {
+  const uint2 where = __ldg(reinterpret_cast<const uint2*>(p.sub_head + n));  // offset16, size16
+  stage_schedule<T>(smeta, p.sub_meta + where.x, where.y & 0xffffu);
+  load_rows_async<NB, T>(src, n, bins, buf0, p.pitch);
+  cp_async_wait_all();
+  __syncthreads();
+  const SubHead& head = *reinterpret_cast<const SubHead*>(smeta);
+  const char* m = smeta + sizeof(SubHead);
+  const int last = static_cast<int>(head.npasses) - (root ? 1 : 0);
+  for (int k = 0; k < last; ++k) {
+    run_pass<NB, T>(head.pass[k], m, buf0, buf1, p.pitch, bins);
+    m += pass_bytes(head.pass[k]);
+    const uint32_t t = buf0;
+    buf0 = buf1;
+    buf1 = t;
+    __syncthreads();
+  }
+  *meta = m;
+  return buf0;
+}
+
+// Column block `hb`: stages its schedule, loads its bottom rows from `src`
+// (scratch that this CTA wrote before its last barrier), evaluates its passes.
+// The output rows end in buf0.
+template <int NB, int T>
+__device__ __forceinline__ void eval_block(const SearchParams& p, const ColBlock& hb, const ColBlock* next, const float* src,
+                           uint32_t bins, uint32_t buf0, uint32_t buf1, char* smeta) {
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t pitch = p.pitch;
-  const uint32_t K = hb.levels;
-  uint32_t nmeta = 0;
-  for (uint32_t k = 0; k < K; ++k) nmeta += hb.count[k];
-  const MetaEntry* gm = p.col_meta + hb.meta;  // 16-byte aligned, padded to an even count
-  for (uint32_t e = 2 * threadIdx.x; e < nmeta; e += 2 * T) cp_async16(cmeta + e, gm + e);
-  float* bottom = (K & 1) ? buf1 : buf0;
-  const uint32_t nb = hb.count[K];
+  stage_schedule<T>(smeta, p.col_meta + hb.meta16, hb.size16);
+  const uint32_t np = hb.npasses;
+  uint32_t from = (np & 1) ? buf1 : buf0, to = (np & 1) ? buf0 : buf1;
+  const uint32_t nb = hb.nbottom;
   const uint32_t nruns = hb.nruns;
   const bool last_ok = lane + 32u * (NB - 1) < bins;
-  // Bottom rows: async copies, all in flight at once.  The rows were written
-  // by other CTAs of the cluster before the cluster barrier, whose acquire
-  // makes them visible to these (L1-allocating) reads.
+  // Bottom rows: async copies, all in flight at once.
   for (uint32_t q = warp; q < nb; q += T / 32) {
     uint32_t j = 0;  // run holding buffer row q (runs ascend in run_off)
 #pragma unroll
     for (uint32_t r = 1; r < 8; ++r) j += (r < nruns && hb.run_off[r] <= q) ? 1u : 0u;
-    const float* g = src + static_cast<uint64_t>(hb.run_row[j] + (q - hb.run_off[j])) * bins + lane;
-    float* o = bottom + q * pitch + lane;
-#pragma unroll
-    for (int i = 0; i < NB; ++i)
-      if (i < NB - 1 || last_ok) cp_async4(o + 32 * i, g + 32 * i);
+    load_row_async<NB>(src + static_cast<uint64_t>(hb.run_row[j] + (q - hb.run_off[j])) * bins, bins,
+                       g_smem + from + q * pitch, lane, last_ok);
   }
   cp_async_wait_all();
   __syncthreads();
-  uint32_t off = 0;
-  for (int k = static_cast<int>(K) - 1; k >= 0; --k) {
-    merge_level<NB, T>(cmeta + off, hb.count[k], ((k + 1) & 1) ? buf1 : buf0, (k & 1) ? buf1 : buf0, pitch, bins);
-    off += hb.count[k];
+  // the next block's rows, from DRAM while this block is evaluated
+  if (next && threadIdx.x < next->nruns) {
+    const uint32_t j = threadIdx.x;
+    const uint32_t n = (j + 1 < next->nruns ? next->run_off[j + 1] : next->nbottom) - next->run_off[j];
+    prefetch_l2(src + static_cast<uint64_t>(next->run_row[j]) * bins, static_cast<uint64_t>(n) * bins);
+  }
+  const char* m = smeta;
+  for (uint32_t k = 0; k < np; ++k) {
+    run_pass<NB, T>(hb.pass[k], m, from, to, pitch, bins);
+    m += pass_bytes(hb.pass[k]);
+    const uint32_t t = from;
+    from = to;
+    to = t;
     __syncthreads();
   }
 }
@@ -623,25 +899,20 @@ __device__ __forceinline__ void load_header(ColBlock* dst, const ColBlock* src) 
     cp_async16(reinterpret_cast<uint4*>(dst) + threadIdx.x, reinterpret_cast<const uint4*>(src) + threadIdx.x);
 }
 
-// One (series, task) per cluster (cluster size 1, 2, 4 or 8); items are
-// task-major so the series of one task run together.  NB = ceil(bins/32)
-// of every task of the launch.
+// One (series, task) per CTA; items are task-major so the series of one task
+// run together.  NB = ceil(bins/32) of every task of the launch.
 template <int NB, int T>
-__global__ void __launch_bounds__(T, T <= 512 ? 2 : 1) ffa_search_kernel(SearchParams p) {
-  cg::cluster_group cluster = cg::this_cluster();
-  const uint32_t cs = cluster.num_blocks();
-  const uint32_t rank = cluster.block_rank();
-  const uint32_t cid = blockIdx.x / cs;
-  const uint32_t nclusters = gridDim.x / cs;
+__global__ void __launch_bounds__(T, T == kSmallThreads ? 2 : 1) ffa_search_kernel(SearchParams p) {
+  __shared__ TrialDev trials[kMaxWidths];
   const uint32_t pitch = p.pitch;
   ColBlock* hdr = reinterpret_cast<ColBlock*>(g_smem);
-  MetaEntry* cmeta = reinterpret_cast<MetaEntry*>(g_smem + 32);
-  float* buf0 = g_smem + p.front;
-  float* buf1 = buf0 + p.max_rows * pitch;
-  float* q0 = p.scratch ? p.scratch + static_cast<uint64_t>(cid) * 2 * p.scratch_elems : nullptr;
-  float* q1 = q0 ? q0 + p.scratch_elems : nullptr;
+  char* smeta = reinterpret_cast<char*>(g_smem + 32);
+  const uint32_t buf0 = p.front;
+  const uint32_t buf1 = buf0 + p.max_rows * pitch;
+  float* q0 = p.scratch ? p.scratch + blockIdx.x * (p.scratch_elems0 + p.scratch_elems1) : nullptr;
+  float* q1 = q0 ? q0 + p.scratch_elems0 : nullptr;
   const uint64_t nitems = p.units ? p.nitems : static_cast<uint64_t>(p.nseries) * p.nitem_tasks;
-  for (uint64_t item = cid; item < nitems; item += nclusters) {
+  for (uint64_t item = blockIdx.x; item < nitems; item += gridDim.x) {
     uint32_t task, series;
     const float* base;
     uint64_t stride;
@@ -666,7 +937,10 @@ __global__ void __launch_bounds__(T, T <= 512 ? 2 : 1) ffa_search_kernel(SearchP
     const TaskDev t = p.tasks[task];
     const float* input = base + series * stride + t.prep_offset;
     const uint32_t bins = t.bins;
-    const DetectArgs da = make_detect(p, t, series, task);
+    // the item's width trials; every path to detection passes a barrier, and so
+    // does the end of the last item's detection
+    for (uint32_t k = threadIdx.x; k < t.ntrials; k += T) trials[k] = p.trials[t.trial_offset + k];
+    const DetectArgs da = make_detect(p, t, trials, series, task);
     const uint32_t cp_pitch = (bins + t.max_width + 2) | 1u;
     const uint32_t dS = t.split_depth;
     if (dS == 0) {
@@ -675,60 +949,78 @@ __global__ void __launch_bounds__(T, T <= 512 ? 2 : 1) ffa_search_kernel(SearchP
         load_rows_async<NB, T>(input, 1, bins, buf0, pitch);
         cp_async_wait_all();
         __syncthreads();
-        detect_rows<NB, T>(buf0, pitch, 1, 0, buf1, cp_pitch, da);
+        detect_rows<NB, T>(g_smem + buf0, pitch, 1, 0, g_smem + buf1, cp_pitch, da);
         __syncthreads();  // the width scans read buf1 until here; the next item loads into it
         continue;
       }
-      float* lvl1 = eval_subtree<NB, T>(p, input, t.rows, bins, 1, buf0, buf1, cmeta);
-      float* other = lvl1 == buf0 ? buf1 : buf0;
-      const uint32_t md = tree_depth(t.rows);
-      const MetaEntry* root = cmeta + (md - 1) * t.rows;
+      const char* root;
+      const uint32_t below = eval_subtree<NB, T>(p, input, t.rows, bins, true, buf0, buf1, smeta, &root);
+      const uint32_t other = below == buf0 ? buf1 : buf0;
+      const SubHead& head = *reinterpret_cast<const SubHead*>(smeta);
+      const uint16_t root_pass = head.pass[head.npasses - 1];
       const uint32_t batch = umin32(T, (p.max_rows * pitch) / (pitch + cp_pitch));
       for (uint32_t b0 = 0; b0 < t.rows_eval; b0 += batch) {
         const uint32_t cnt = umin32(batch, t.rows_eval - b0);
-        merge_level<NB, T>(root + b0, cnt, lvl1, other, pitch, bins);
+        merge_rows<NB, T>(root_pass, root, below, other, pitch, bins, b0, b0 + cnt);
         __syncthreads();
-        detect_rows<NB, T>(other, pitch, cnt, b0, other + batch * pitch, cp_pitch, da);
+        detect_rows<NB, T>(g_smem + other, pitch, cnt, b0, g_smem + other + batch * pitch, cp_pitch, da);
       }
       __syncthreads();  // the last width scans read `other` until here; the next item loads into it
       continue;
     }
-    // 1. subtrees at depth dS, on chip, into scratch q0
-    const uint32_t nsub = 1u << dS;
-    for (uint32_t sub = rank; sub < nsub; sub += cs) {
-      const Node nd = node_at(sub, t.rows, dS);
-      const float* res = eval_subtree<NB, T>(p, input + static_cast<uint64_t>(nd.a) * bins, nd.n, bins, 0, buf0, buf1,
-                                          cmeta);
-      store_rows<NB, T>(res, pitch, nd.n, bins, q0 + static_cast<uint64_t>(nd.a) * bins);
-      __syncthreads();
-    }
-    cluster.sync();
-    // 2. column passes up to the root (the last one fused with detection)
-    float* src = q0;
-    float* dst = q1;
+    // Subtrees at depth dS on chip, then column passes up to the root (the last
+    // one fused with detection).  The first pass follows the subtrees node by
+    // node: a node of depth first_depth is at most 8 subtrees, whose rows (well
+    // under 1 MB) it reads back from L2 right after they are written there,
+    // into scratch that the next node uses again (all subtrees first: 47.4 ms
+    // on the survey plan, 45.9 node by node).
+    uint32_t block = 0;  // next block of the pass
     for (uint32_t ps = 0; ps < t.npasses; ++ps) {
       const PassDev pd = p.passes[t.pass_begin + ps];
       const ColBlock* blocks = p.blocks + pd.block_begin;
-      if (rank < pd.nblocks) load_header(&hdr[0], blocks + rank);
-      cp_async_wait_all();
-      __syncthreads();
-      uint32_t it = 0;
-      for (uint32_t u = rank; u < pd.nblocks; u += cs, ++it) {
-        const ColBlock& hb = hdr[it & 1];
-        if (u + cs < pd.nblocks) load_header(&hdr[(it + 1) & 1], blocks + u + cs);
-        eval_block<NB, T>(p, hb, src, bins, buf0, buf1, cmeta);
-        if (hb.final_pass) {
-          detect_rows<NB, T>(buf0, pitch, hb.count[0], hb.out_row, buf1, cp_pitch, da);
-          __syncthreads();  // the width scans read buf1 until here; the next block may load into it
-        } else {
-          store_rows<NB, T>(buf0, pitch, hb.count[0], bins, dst + static_cast<uint64_t>(hb.out_row) * bins);
-          __syncthreads();
+      const uint32_t nnodes = ps == 0 ? 1u << t.first_depth : 1u;
+      const float* src = (ps & 1) ? q1 : q0;
+      float* dst = (ps & 1) ? q0 : q1;
+      block = 0;
+      for (uint32_t node = 0; node < nnodes; ++node) {
+        uint32_t end = pd.nblocks;
+        if (ps == 0) {
+          const Node X = node_at(node, t.rows, t.first_depth);
+          const uint32_t per = 1u << (dS - t.first_depth);
+          for (uint32_t sub = node * per; sub < (node + 1) * per; ++sub) {
+            const Node nd = node_at(sub, t.rows, dS);
+            if (threadIdx.x == 0 && nd.a + nd.n < t.rows)
+              prefetch_l2(input + static_cast<uint64_t>(nd.a + nd.n) * bins,
+                          umin64(nd.n, t.rows - nd.a - nd.n) * bins);
+            const char* meta_end;
+            const uint32_t res = eval_subtree<NB, T>(p, input + static_cast<uint64_t>(nd.a) * bins, nd.n, bins, false,
+                                                     buf0, buf1, smeta, &meta_end);
+            store_rows<NB, T>(res, pitch, nd.n, bins, q0 + static_cast<uint64_t>(nd.a - X.a) * bins);
+            __syncthreads();
+          }
+          src = q0 - static_cast<uint64_t>(X.a) * bins;
+          if (t.first_depth > 0) end = block + (X.n + p.block_rows - 1) / p.block_rows;
+        }
+        if (block < end) load_header(&hdr[block & 1], blocks + block);
+        cp_async_wait_all();
+        __syncthreads();
+        for (; block < end; ++block) {
+          const ColBlock& hb = hdr[block & 1];
+          const ColBlock* next = nullptr;
+          if (block + 1 < end) {
+            load_header(&hdr[(block + 1) & 1], blocks + block + 1);
+            next = &hdr[(block + 1) & 1];
+          }
+          eval_block<NB, T>(p, hb, next, src, bins, buf0, buf1, smeta);
+          if (hb.final_pass) {
+            detect_rows<NB, T>(g_smem + buf0, pitch, hb.rows, hb.out_row, g_smem + buf1, cp_pitch, da);
+            __syncthreads();  // the width scans read buf1 until here; the next block may load into it
+          } else {
+            store_rows<NB, T>(buf0, pitch, hb.rows, bins, dst + static_cast<uint64_t>(hb.out_row) * bins);
+            __syncthreads();
+          }
         }
       }
-      cluster.sync();
-      float* tmp = src;
-      src = dst;
-      dst = tmp;
     }
   }
 }
@@ -791,13 +1083,12 @@ struct FfaGeometry {
 };
 
 struct FfaClass {
-  int cluster = 1;             // CTAs cooperating on one (series, task)
   int threads = kThreads;      // CTA size (kSmallThreads or kThreads)
   uint32_t nb = 1;             // ceil(bins / 32) of every task of the class
   SearchKernel kernel = nullptr;
   std::vector<uint32_t> tasks; // largest first
-  uint64_t max_elems = 0;      // rows * bins of the largest task (scratch per cluster)
-  int nclusters = 0;           // resident clusters
+  uint64_t scratch0 = 0, scratch1 = 0;  // scratch floats per CTA: subtree rows, pass outputs
+  int nctas = 0;               // resident CTAs
   DeviceBlob tasks_d;
   std::vector<UnitDev> units;  // batched programs: one item run per task, in task order
   uint64_t nitems = 0;
@@ -826,9 +1117,9 @@ struct gf_ffa_program {
   std::vector<FfaMember> members;
   std::vector<TaskDev> task_dev;
   std::vector<TrialDev> trial_dev;
-  std::vector<MetaEntry> sub_meta;
-  std::vector<uint32_t> sub_offset;
-  std::vector<MetaEntry> col_meta;
+  std::vector<uint4> sub_meta;
+  std::vector<SubHead> sub_head;
+  std::vector<uint4> col_meta;
   std::vector<ColBlock> blocks;
   std::vector<PassDev> passes;
   std::vector<FfaClass> classes;
@@ -836,7 +1127,7 @@ struct gf_ffa_program {
   FfaGeometry geo[2][17];      // by CTA size (0: kSmallThreads, 1: kThreads) and NB (1..16)
   uint64_t max_series = 0;
   uint64_t scratch_floats = 0;
-  DeviceBlob tasks_d, trials_d, sub_meta_d, sub_offset_d, col_meta_d, blocks_d, passes_d, members_d;
+  DeviceBlob tasks_d, trials_d, sub_meta_d, sub_head_d, col_meta_d, blocks_d, passes_d, members_d;
   // batched prepare of every member (gf_ffa_batch_bind_series)
   DeviceBlob prepare_items_d, prepare_begin_d;
   uint64_t prepare_ctas_total = 0, prepare_halo = 0;
@@ -895,12 +1186,102 @@ uint32_t host_tree_depth(uint64_t n) {
   return d;
 }
 
-// Merge schedule of a subtree of n rows (ffa.cpp:127-195 recursion, by
-// depth): for level l = depth-1 .. 0 and each row r, either MERGE(head row,
+// Groups of the rows `out` (entries over the rows of `mid`, themselves entries
+// over the rows two levels down) into QuadOps, in row order.
+void build_quads(const std::vector<MetaEntry>& out, const std::vector<MetaEntry>& mid, std::vector<QuadOp>& ops) {
+  const size_t n = out.size();
+  auto merged = [&](size_t r) { return mid[r].op == kMerge; };
+  // rows x and y of `mid` share both their inputs, y one phase on
+  auto shared = [&](size_t x, size_t y) {
+    return mid[x].a == mid[y].a && mid[x].b == mid[y].b && mid[y].roll == mid[x].roll + 1;
+  };
+  QuadOp q{};
+  auto head = [&](int i, uint16_t row) {
+    q.a[i] = mid[row].a;
+    q.b[i] = mid[row].b;
+    q.rb[i] = mid[row].roll;
+  };
+  auto tail = [&](int i, uint16_t row, uint16_t roll) {
+    q.c[i] = mid[row].a;
+    q.d[i] = mid[row].b;
+    q.rc[i] = roll;
+    q.rd[i] = static_cast<uint16_t>(roll + mid[row].roll);
+  };
+  for (size_t i = 0; i < n;) {
+    q = QuadOp{};
+    q.row = static_cast<uint16_t>(i);
+    const MetaEntry* o = out.data() + i;
+    auto all_merge = [&](size_t count) {
+      if (i + count > n) return false;
+      for (size_t j = 0; j < count; ++j)
+        if (o[j].op != kMerge || !merged(o[j].a) || !merged(o[j].b)) return false;
+      return true;
+    };
+    if (all_merge(4) && o[0].a == o[1].a && o[2].a == o[3].a) {
+      const int r1 = o[1].roll - o[0].roll, r2 = o[2].roll - o[0].roll, r3 = o[3].roll - o[0].roll;
+      const bool heads = shared(o[0].a, o[2].a);
+      head(0, o[0].a);
+      head(1, o[2].a);
+      if (o[0].b == o[1].b && o[2].b == o[3].b && r1 == 1 && r2 == 1 && r3 == 2) {
+        tail(0, o[0].b, o[0].roll);
+        tail(1, o[2].b, o[2].roll);
+        q.type = heads && shared(o[0].b, o[2].b) ? kOpRS : kOpR;
+        ops.push_back(q);
+        i += 4;
+        continue;
+      }
+      if (o[1].b == o[2].b && r1 == 0 && r2 == 1 && r3 == 1) {
+        tail(0, o[0].b, o[0].roll);
+        tail(1, o[1].b, o[1].roll);
+        tail(2, o[3].b, o[3].roll);
+        q.type = heads ? kOpFS : kOpF;
+        ops.push_back(q);
+        i += 4;
+        continue;
+      }
+    }
+    if (all_merge(2) && o[0].a == o[1].a && o[0].b == o[1].b && o[1].roll == o[0].roll + 1) {
+      head(0, o[0].a);
+      tail(0, o[0].b, o[0].roll);
+      q.type = kOpPair;
+      ops.push_back(q);
+      i += 2;
+      continue;
+    }
+    q.type = kOpOne;
+    head(0, o[0].a);
+    if (merged(o[0].a)) q.flags |= 1;
+    if (o[0].op == kMerge) {
+      tail(0, o[0].b, o[0].roll);
+      q.flags |= merged(o[0].b) ? 6 : 2;
+    }
+    ops.push_back(q);
+    ++i;
+  }
+}
+
+// Appends a pass's entries to `meta` (16-byte words); returns its descriptor.
+uint16_t append_pass(const std::vector<QuadOp>& ops, std::vector<uint4>& meta) {
+  const size_t at = meta.size();
+  meta.resize(at + 3 * ops.size());
+  std::memcpy(meta.data() + at, ops.data(), ops.size() * sizeof(QuadOp));
+  return static_cast<uint16_t>(kPassTwo | ops.size());
+}
+uint16_t append_pass(const std::vector<MetaEntry>& entries, std::vector<uint4>& meta) {
+  const size_t at = meta.size();
+  meta.resize(at + (entries.size() + 1) / 2);
+  std::memcpy(meta.data() + at, entries.data(), entries.size() * sizeof(MetaEntry));
+  return static_cast<uint16_t>(entries.size());
+}
+
+// The merges of a subtree of n rows (ffa.cpp:127-195 recursion, by depth):
+// level[l][r] for l = depth-1 .. 0 and each row r is either MERGE(head row,
 // tail row, roll) from level l+1 or CARRY(r) for rows of one-row nodes.
-void build_subtree_schedule(uint32_t n, std::vector<MetaEntry>& out) {
+std::vector<std::vector<MetaEntry>> subtree_levels(uint32_t n) {
   const uint32_t md = host_tree_depth(n);
+  std::vector<std::vector<MetaEntry>> level(md);
   for (int l = static_cast<int>(md) - 1; l >= 0; --l) {
+    std::vector<MetaEntry>& out = level[l];
     for (uint32_t r = 0; r < n; ++r) {
       uint32_t a = 0, sz = n, depth = 0;
       while (depth < static_cast<uint32_t>(l) && sz > 1) {
@@ -928,6 +1309,28 @@ void build_subtree_schedule(uint32_t n, std::vector<MetaEntry>& out) {
       out.push_back(m);
     }
   }
+  return level;
+}
+
+// Schedule of a subtree: the odd level out by itself at the leaves (mostly
+// carries there), then two levels per pass up to the root.
+SubHead build_subtree_schedule(uint32_t n, std::vector<uint4>& meta) {
+  SubHead h{};
+  h.offset16 = static_cast<uint32_t>(meta.size());
+  meta.resize(meta.size() + sizeof(SubHead) / 16);
+  const auto level = subtree_levels(n);
+  int l = static_cast<int>(level.size());
+  if (l & 1) h.pass[h.npasses++] = append_pass(level[--l], meta);
+  while (l > 0) {
+    std::vector<QuadOp> ops;
+    build_quads(level[l - 2], level[l - 1], ops);
+    check_arg(h.npasses < kMaxPasses, "FFA subtree too deep");
+    h.pass[h.npasses++] = append_pass(ops, meta);
+    l -= 2;
+  }
+  h.size16 = static_cast<uint16_t>(meta.size() - h.offset16);
+  std::memcpy(meta.data() + h.offset16, &h, sizeof h);
+  return h;
 }
 
 // Pass boundaries: depth cuts from split_depth down to 0, K levels per pass;
@@ -957,13 +1360,12 @@ struct ColumnNode {
 // tail-child rows its rows read (the index arithmetic of ffa.cpp), so each
 // level stays within max_rows rows.
 void build_column_block(uint32_t bins, uint32_t xa, uint32_t xn, uint32_t s0, uint32_t s1, uint32_t K,
-                        uint32_t max_rows, bool final_pass, std::vector<MetaEntry>& meta,
+                        uint32_t max_rows, uint32_t meta_bytes, bool final_pass, std::vector<uint4>& meta,
                         std::vector<ColBlock>& blocks) {
   ColBlock b{};
-  b.levels = static_cast<uint8_t>(K);
   b.final_pass = final_pass ? 1 : 0;
   b.out_row = final_pass ? s0 : xa + s0;
-  b.count[0] = static_cast<uint16_t>(s1 - s0);
+  b.rows = static_cast<uint16_t>(s1 - s0);
   std::vector<ColumnNode> nodes{ColumnNode{xa, xn, s0, s1, 0}};
   std::vector<std::vector<MetaEntry>> level(K);
   for (uint32_t k = 0; k < K; ++k) {
@@ -992,7 +1394,7 @@ void build_column_block(uint32_t bins, uint32_t xa, uint32_t xn, uint32_t s0, ui
     check_arg(off <= max_rows, "FFA column schedule exceeds the shared-memory tile");
     for (const MetaEntry& m : level[k])
       check_arg(m.a < off && m.b < off && m.roll < bins, "FFA column schedule entry out of range");
-    b.count[k + 1] = static_cast<uint16_t>(off);
+    b.nbottom = static_cast<uint16_t>(off);
     nodes.swap(children);
   }
   check_arg(nodes.size() <= 8, "FFA column block has too many bottom runs");
@@ -1002,10 +1404,27 @@ void build_column_block(uint32_t bins, uint32_t xa, uint32_t xn, uint32_t s0, ui
     b.run_off[j] = static_cast<uint16_t>(nodes[j].off);
     b.run_row[j] = static_cast<uint16_t>(nodes[j].a + nodes[j].u0);
   }
-  if (meta.size() & 1) meta.push_back(MetaEntry{});
-  b.meta = static_cast<uint32_t>(meta.size());
-  for (int k = static_cast<int>(K) - 1; k >= 0; --k) meta.insert(meta.end(), level[k].begin(), level[k].end());
-  if (meta.size() & 1) meta.push_back(MetaEntry{});
+  // two levels per pass from the bottom, an odd one by itself at the top (the
+  // level of the fewest rows); one level at a time where the staged schedule
+  // would not hold the groups
+  b.meta16 = static_cast<uint32_t>(meta.size());
+  for (bool two : {true, false}) {
+    meta.resize(b.meta16);
+    b.npasses = 0;
+    for (int k = static_cast<int>(K); k > 0;) {
+      if (two && k >= 2) {
+        std::vector<QuadOp> ops;
+        build_quads(level[k - 2], level[k - 1], ops);
+        b.pass[b.npasses++] = append_pass(ops, meta);
+        k -= 2;
+      } else {
+        b.pass[b.npasses++] = append_pass(level[--k], meta);
+      }
+    }
+    if ((meta.size() - b.meta16) * 16 <= meta_bytes) break;
+  }
+  check_arg((meta.size() - b.meta16) * 16 <= meta_bytes, "FFA column schedule exceeds its staging area");
+  b.size16 = static_cast<uint16_t>(meta.size() - b.meta16);
   blocks.push_back(b);
 }
 
@@ -1032,9 +1451,11 @@ void build_task_passes(gf_ffa_program& P, const FfaGeometry& g, TaskDev& d) {
       const uint32_t s0 = (u % bpn) * R;
       const uint32_t s1 = std::min<uint32_t>(s0 + R, final_pass ? d.rows_eval : X.n);
       if (s0 >= s1) continue;
-      build_column_block(d.bins, X.a, X.n, s0, s1, levels, g.max_rows, final_pass, P.col_meta, P.blocks);
+      build_column_block(d.bins, X.a, X.n, s0, s1, levels, g.max_rows, (g.front - 32) * 4, final_pass, P.col_meta,
+                         P.blocks);
     }
     pd.nblocks = static_cast<uint32_t>(P.blocks.size()) - pd.block_begin;
+    if (depth == dS) d.first_depth = dn;
     P.passes.push_back(pd);
     if (final_pass) break;
     depth = dn;
@@ -1074,6 +1495,14 @@ struct MemberSpec {
   uint64_t nwidths;
   uint64_t nseries;
 };
+
+// The same limit for every program, whatever its own tiles: programs of
+// several threads share the kernels, and a lower limit would fail a launch.
+void set_search_smem(const FfaClass& c) {
+  cuda_check(cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(c.threads == kSmallThreads ? kSmallSmem : kLargeSmem)),
+             "cudaFuncSetAttribute(ffa_search_kernel)");
+}
 
 // Tables of every member's tasks: octaves, boxcar trials, on-chip geometry,
 // column schedules and the launch classes.  Batched programs also get one
@@ -1127,19 +1556,29 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
   // staged schedule, two row buffers of max_rows rows of the class's widest
   // rows; sized for two 512-thread CTAs or one 1024-thread CTA per SM (227 KB
   // per CTA at most, static state aside)
-  uint32_t max_rows_all = 0;
+  // subtree schedules of every size, built as far as the tiles need them;
+  // sub_bytes[n]: the most that a size up to n stages
+  std::vector<uint32_t> sub_bytes{0u};
+  P->sub_head.push_back(SubHead{});
+  auto schedules_to = [&](uint32_t n) {
+    while (P->sub_head.size() <= n) {
+      P->sub_head.push_back(build_subtree_schedule(static_cast<uint32_t>(P->sub_head.size()), P->sub_meta));
+      sub_bytes.push_back(std::max(sub_bytes.back(), 16u * P->sub_head.back().size16));
+    }
+    return sub_bytes[n];
+  };
   for (int gi = 0; gi < 2; ++gi)
   for (uint32_t nb = 1; nb <= 16; ++nb) {
-    const size_t budget = gi == 0 ? 110 * 1024 : 222 * 1024;
+    const size_t budget = gi == 0 ? kSmallSmem : kLargeSmem;
     FfaGeometry& g = P->geo[gi][nb];
     const uint32_t cap = std::min<uint32_t>(32 * nb, P->max_bins);
     if (32 * (nb - 1) >= P->max_bins) break;
-    g.pitch = cap | 1u;
+    g.pitch = (cap + kHalo) | 1u;
     g.levels = 3;
     auto front_for = [&](uint32_t rows) {
-      const uint64_t meta_cap = std::max<uint64_t>(static_cast<uint64_t>(tree_depth(rows)) * rows,
-                                                   static_cast<uint64_t>(g.levels) * rows + 2);
-      return static_cast<uint32_t>(round_up(std::max<uint64_t>(32 + 2 * meta_cap, cap), 4));
+      // the largest subtree, or a column block taken one level at a time
+      const uint64_t meta_cap = std::max<uint64_t>(schedules_to(rows), g.levels * (8ull * rows + 16));
+      return static_cast<uint32_t>(round_up(std::max<uint64_t>(32 + meta_cap / 4, cap), 4));
     };
     auto smem_for = [&](uint32_t rows) { return (front_for(rows) + 2ull * rows * g.pitch) * 4; };
     uint32_t rows = 8;
@@ -1154,16 +1593,8 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
     g.final_rows = std::min<uint32_t>(g.block_rows, g.cp_rows);
     check_arg(g.final_rows >= 1 && g.block_rows >= 1, "FFA bins too large for the shared-memory tiles");
     g.smem_bytes = smem_for(rows);
-    max_rows_all = std::max(max_rows_all, rows);
   }
-  const uint32_t rows = max_rows_all;
-  // subtree schedules for every size up to max_rows
-  P->sub_offset.assign(rows + 1, 0u);
-  for (uint32_t n = 1; n <= rows; ++n) {
-    P->sub_offset[n] = static_cast<uint32_t>(P->sub_meta.size());
-    build_subtree_schedule(n, P->sub_meta);
-  }
-  if (P->sub_meta.empty()) P->sub_meta.push_back(MetaEntry{});
+  if (P->sub_meta.empty()) P->sub_meta.resize(1);
   // tasks, trials, column schedules and classes
   std::map<std::tuple<int, uint32_t, int>, size_t> class_of;
   for (uint64_t i = 0; i < P->tasks.size(); ++i) {
@@ -1200,31 +1631,28 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
     d.split_depth = ds;
     if (ds > 0) build_task_passes(*P, g, d);
     P->task_dev.push_back(d);
-    // cluster sized by rows for split tasks; on-chip tasks use key 0
-    int cluster = 1;
-    if (ds > 0) {
-      while (cluster < kClusterSize && static_cast<uint64_t>(cluster) * 512 < t.rows) cluster *= 2;
-    }
     const uint32_t nb = static_cast<uint32_t>(ceil_div(t.bins, 32));
     const int threads = gi == 0 ? kSmallThreads : kThreads;
-    const std::tuple<int, uint32_t, int> key{ds == 0 ? 0 : cluster, nb, threads};
+    const std::tuple<int, uint32_t, int> key{ds == 0 ? 0 : 1, nb, threads};
     if (!class_of.count(key)) {
       class_of[key] = P->classes.size();
       P->classes.emplace_back();
-      P->classes.back().cluster = cluster;
       P->classes.back().threads = threads;
       P->classes.back().nb = nb;
       P->classes.back().kernel = search_kernel_for(nb, threads);
     }
     FfaClass& c = P->classes[class_of[key]];
     c.tasks.push_back(static_cast<uint32_t>(i));
-    if (ds > 0) c.max_elems = std::max<uint64_t>(c.max_elems, t.rows * t.bins);
+    if (ds > 0) {
+      // subtree rows of one first-pass node; a third pass writes whole tasks there too
+      const uint64_t node_rows = ceil_div(t.rows, 1ull << d.first_depth);
+      c.scratch0 = std::max<uint64_t>(c.scratch0, (d.npasses > 2 ? t.rows : node_rows) * t.bins);
+      if (d.npasses > 1) c.scratch1 = std::max<uint64_t>(c.scratch1, t.rows * t.bins);
+    }
   }
-  // launch order: widest clusters (longest items) first
-  std::stable_sort(P->classes.begin(), P->classes.end(), [](const FfaClass& x, const FfaClass& y) {
-    return x.cluster != y.cluster ? x.cluster > y.cluster : x.nb > y.nb;
-  });
-  if (P->col_meta.empty()) P->col_meta.resize(2);
+  std::stable_sort(P->classes.begin(), P->classes.end(),
+                   [](const FfaClass& x, const FfaClass& y) { return x.nb > y.nb; });
+  if (P->col_meta.empty()) P->col_meta.resize(1);
   if (P->blocks.empty()) P->blocks.resize(1);
   if (P->passes.empty()) P->passes.resize(1);
   for (auto& c : P->classes) {
@@ -1241,36 +1669,24 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
       c.units_d.upload(c.units.data(), c.units.size() * sizeof(UnitDev), device_id);
     }
     const FfaGeometry& g = P->geo[c.threads == kSmallThreads ? 0 : 1][c.nb];
-    cuda_check(cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(g.smem_bytes)),
-               "cudaFuncSetAttribute(ffa_search_kernel)");
-    cuda_check(cudaFuncSetAttribute(c.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-               "cudaFuncSetAttribute(cluster size)");
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(c.cluster, 1, 1);
-    cfg.blockDim = dim3(static_cast<unsigned>(c.threads), 1, 1);
-    cfg.dynamicSmemBytes = g.smem_bytes;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = c.cluster;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    set_search_smem(c);
     int n = 0;
-    cuda_check(cudaOccupancyMaxActiveClusters(&n, c.kernel, &cfg), "cudaOccupancyMaxActiveClusters");
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, c.kernel, c.threads, g.smem_bytes),
+               "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     check_arg(n > 0, "FFA kernel cannot be resident on this device");
-    c.nclusters = n;
+    int sms = 0;
+    cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_id), "cudaDeviceGetAttribute");
+    c.nctas = n * sms;
     // classes run one after another on the stream: they share the scratch
-    P->scratch_floats = std::max<uint64_t>(P->scratch_floats, static_cast<uint64_t>(n) * 2 * c.max_elems);
+    P->scratch_floats = std::max<uint64_t>(P->scratch_floats, static_cast<uint64_t>(c.nctas) * (c.scratch0 + c.scratch1));
     c.tasks_d.upload(c.tasks.data(), c.tasks.size() * sizeof(uint32_t), device_id);
   }
   P->tasks_d.upload(P->task_dev.data(), P->task_dev.size() * sizeof(TaskDev), device_id);
   P->trials_d.upload(P->trial_dev.data(), P->trial_dev.size() * sizeof(TrialDev), device_id);
   for (auto& M : P->members) M.octaves_d.upload(M.octaves.data(), M.octaves.size() * sizeof(OctaveDev), device_id);
-  P->sub_meta_d.upload(P->sub_meta.data(), P->sub_meta.size() * sizeof(MetaEntry), device_id);
-  P->sub_offset_d.upload(P->sub_offset.data(), P->sub_offset.size() * sizeof(uint32_t), device_id);
-  P->col_meta_d.upload(P->col_meta.data(), P->col_meta.size() * sizeof(MetaEntry), device_id);
+  P->sub_meta_d.upload(P->sub_meta.data(), P->sub_meta.size() * sizeof(uint4), device_id);
+  P->sub_head_d.upload(P->sub_head.data(), P->sub_head.size() * sizeof(SubHead), device_id);
+  P->col_meta_d.upload(P->col_meta.data(), P->col_meta.size() * sizeof(uint4), device_id);
   P->blocks_d.upload(P->blocks.data(), P->blocks.size() * sizeof(ColBlock), device_id);
   P->passes_d.upload(P->passes.data(), P->passes.size() * sizeof(PassDev), device_id);
   return P;
@@ -1334,15 +1750,15 @@ void launch_search(gf_ffa_program* P, const float* dev_prepared, uint64_t nserie
   sp.prep_stride = P->members[0].prep_stride;
   sp.tasks = P->tasks_d.as<TaskDev>();
   sp.trials = P->trials_d.as<TrialDev>();
-  sp.sub_meta = P->sub_meta_d.as<MetaEntry>();
-  sp.sub_offset = P->sub_offset_d.as<uint32_t>();
+  sp.sub_meta = P->sub_meta_d.as<uint4>();
+  sp.sub_head = P->sub_head_d.as<SubHead>();
   sp.nseries = static_cast<uint32_t>(nseries);
   sp.members = P->batched ? P->members_d.as<MemberDev>() : nullptr;
   sp.threshold = snr_threshold;
   sp.peaks = dev_peaks;
   sp.capacity = capacity;
   sp.counters = reinterpret_cast<unsigned long long*>(dev_counters);
-  sp.col_meta = P->col_meta_d.as<MetaEntry>();
+  sp.col_meta = P->col_meta_d.as<uint4>();
   sp.blocks = P->blocks_d.as<ColBlock>();
   sp.passes = P->passes_d.as<PassDev>();
   sp.scratch = static_cast<float*>(dev_scratch);
@@ -1352,27 +1768,19 @@ void launch_search(gf_ffa_program* P, const float* dev_prepared, uint64_t nserie
     sp.units = P->batched ? c.units_d.as<UnitDev>() : nullptr;
     sp.nunits = static_cast<uint32_t>(c.units.size());
     sp.nitems = c.nitems;
-    sp.scratch_elems = c.max_elems;
+    sp.scratch_elems0 = c.scratch0;
+    sp.scratch_elems1 = c.scratch1;
     const FfaGeometry& g = P->geo[c.threads == kSmallThreads ? 0 : 1][c.nb];
     sp.pitch = g.pitch;
     sp.max_rows = g.max_rows;
     sp.front = g.front;
+    sp.block_rows = g.block_rows;
     const uint64_t items = P->batched ? c.nitems : nseries * c.tasks.size();
     if (items == 0) continue;
-    const unsigned nclusters = static_cast<unsigned>(std::min<uint64_t>(items, static_cast<uint64_t>(c.nclusters)));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nclusters * c.cluster, 1, 1);
-    cfg.blockDim = dim3(static_cast<unsigned>(c.threads), 1, 1);
-    cfg.dynamicSmemBytes = g.smem_bytes;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = c.cluster;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cuda_check(cudaLaunchKernelEx(&cfg, c.kernel, sp), "ffa_search_kernel launch");
+    const unsigned ctas = static_cast<unsigned>(std::min<uint64_t>(items, static_cast<uint64_t>(c.nctas)));
+    set_search_smem(c);
+    c.kernel<<<ctas, static_cast<unsigned>(c.threads), g.smem_bytes, s>>>(sp);
+    cuda_check(cudaGetLastError(), "ffa_search_kernel launch");
   }
 }
 
@@ -1470,7 +1878,7 @@ extern "C" int gf_ffa_program_info(const gf_ffa_program* P, gf_ffa_info* info) {
     uint64_t mx = 0;
     for (const auto& t : P->tasks) mx = std::max<uint64_t>(mx, t.rows * t.bins);
     info->max_task_elements = mx;
-    info->metadata_bytes = P->tasks_d.bytes + P->trials_d.bytes + P->sub_meta_d.bytes + P->sub_offset_d.bytes +
+    info->metadata_bytes = P->tasks_d.bytes + P->trials_d.bytes + P->sub_meta_d.bytes + P->sub_head_d.bytes +
                            P->col_meta_d.bytes + P->blocks_d.bytes + P->passes_d.bytes + P->members_d.bytes;
     for (const auto& M : P->members) info->metadata_bytes += M.octaves_d.bytes;
     for (const auto& c : P->classes) info->metadata_bytes += c.tasks_d.bytes + c.units_d.bytes;
