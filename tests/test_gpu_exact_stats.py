@@ -1,0 +1,58 @@
+"""Statistics of detrended series: the parallel FP64 sums must have the bits of
+the sequential loop, on series whose sums are all exact, exact up to some
+segment (16384 samples), never exact, and not finite."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def sequential_stats(y):
+    y = y.astype(np.float64)
+    total, sq = np.cumsum(y)[-1], np.cumsum(y * y)[-1]     # cumsum adds one by one
+    n = float(len(y))
+    mean = total / n
+    var = sq / n - mean * mean
+    return mean, 1.0 / np.sqrt(var)
+
+
+def series(kind, n, rng):
+    if kind == "u32":                                      # dedispersed sums: exact throughout
+        return (rng.normal(size=n) * 256 + 32768).round().astype(np.int32)
+    if kind == "loud":                                     # sums of squares outgrow 53 bits part way
+        return (rng.normal(size=n) * 20000 + 600000).round().astype(np.int32)
+    return (rng.normal(size=n) * 3).astype(np.float32)     # 24 bits per sample: rounds at once
+
+
+@pytest.mark.parametrize("kind", ["u32", "loud", "f32"])
+@pytest.mark.parametrize("n,stride", [(16384 * 2, 16384 * 2), (16384 * 3 + 5, 16384 * 3 + 8), (40003, 40003),
+                                      (5000, 5003), (16383, 16384)])
+def test_stats_have_the_sequential_bits(kind, n, stride):
+    from gaffa_b200 import core
+    rng = np.random.default_rng(n)
+    x = np.stack([np.resize(series(kind, n, rng), stride) for _ in range(3)])
+    pre = core.PreprocessProgram(n, 1e-3, window_seconds=0.5, min_points=101, max_series=3)
+    t = torch.from_numpy(x).cuda()
+    stats = pre.run(t).cpu().numpy()
+    pre.synchronize()
+    y = t.view(torch.float32).cpu().numpy()[:, :n]
+    for got, row in zip(stats, y):
+        assert tuple(got) == sequential_stats(row)
+
+
+def test_nonfinite_after_an_exact_segment():
+    from gaffa_b200 import core
+    x = np.random.default_rng(1).normal(size=(1, 50000)).astype(np.float32)
+    x[0, 40000] = np.inf
+    pre = core.PreprocessProgram(50000, 1e-3, window_seconds=0.5, min_points=101, max_series=1)
+    pre.run(torch.from_numpy(x).cuda())
+    with pytest.raises(ValueError, match="finite"):
+        pre.synchronize()
