@@ -56,3 +56,19 @@ def test_nonfinite_after_an_exact_segment():
     pre.run(torch.from_numpy(x).cuda())
     with pytest.raises(ValueError, match="finite"):
         pre.synchronize()
+
+
+@pytest.mark.parametrize("w", [1, 3, 5, 63, 101, 127, 129, 255])
+@pytest.mark.parametrize("n", [600, 513, 2049])
+def test_running_median_at_every_window_form(w, n):
+    """Selected (to 127 samples) and sliding medians of an edge-padded series."""
+    from gaffa_b200 import core
+    rng = np.random.default_rng(w * n)
+    x = np.stack([rng.normal(size=n), rng.integers(-3, 4, size=n), np.linspace(-1e6, 1e6, n)]).astype(np.float32)
+    pre = core.PreprocessProgram(n, 1.0, window_seconds=float(w), min_points=w, max_series=3, reject_constant=False)
+    assert int(pre.info.scrunch_factor) == 1
+    t = torch.from_numpy(x.copy()).cuda()
+    pre.run(t)
+    padded = np.pad(x, ((0, 0), (w // 2, w // 2)), mode="edge")
+    med = np.median(np.lib.stride_tricks.sliding_window_view(padded, w, axis=1), axis=2).astype(np.float32)
+    assert np.array_equal(t.cpu().numpy(), x - med)
