@@ -108,8 +108,9 @@ class DmSearch:
             per_dm = self.out_stride * 4 + plan.prepared_floats * 4
             budget = int(free * 0.45) - self.dedisp.info.staged_bytes - (1 << 30)
             dm_batch = max(g, min(ndm, budget // max(1, per_dm)))
-        dm_batch = max(g, (dm_batch // g) * g)
-        self.dm_batch = min(dm_batch, ((ndm + g - 1) // g) * g)
+        # all DMs in one batch where they fit (a ragged last batch would cost a
+        # second round of launches and host steps), else whole blocks of DMs
+        self.dm_batch = ndm if dm_batch >= ndm else max(g, (dm_batch // g) * g)
         self.pre = core.PreprocessProgram(self.nout, tsamp, window_seconds=window_seconds, min_points=min_points,
                                           normalise=True, reject_constant=True, max_series=self.dm_batch,
                                           device_id=device_id)
