@@ -650,12 +650,16 @@ def select_candidates(peaks: np.ndarray, observation_seconds: float, frequency_c
     o = _lib.CandidateOptions(frequency_cluster_radius, dm_cluster_radius, int(cluster_across_widths), 0,
                               max_candidates)
     n = _lib.u64()
-    check(_lib.lib().gf_select_candidates(ptr(peaks), len(peaks), observation_seconds, C.byref(o), None, 0,
-                                          C.byref(n)))
-    out = np.zeros(n.value, _lib.CAND_DTYPE)
-    check(_lib.lib().gf_select_candidates(ptr(peaks), len(peaks), observation_seconds, C.byref(o), ptr(out),
-                                          len(out), C.byref(n)))
-    return out
+    # usually far fewer candidates than peaks: a bounded first guess, and a
+    # second selection only when the candidates exceed it
+    out = np.zeros(min(len(peaks), 1 << 14), _lib.CAND_DTYPE)
+    for _ in range(2):
+        check(_lib.lib().gf_select_candidates(ptr(peaks), len(peaks), observation_seconds, C.byref(o),
+                                              ptr(out) if len(out) else None, len(out), C.byref(n)))
+        if n.value <= len(out):
+            break
+        out = np.zeros(n.value, _lib.CAND_DTYPE)
+    return out[: n.value].copy()
 
 
 def select_candidates_device(program: "FfaProgram", records: torch.Tensor, segments, dm_low: float, dm_step: float,

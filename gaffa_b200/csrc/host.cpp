@@ -9,6 +9,7 @@
 #include <cstring>
 #include <limits>
 #include <numeric>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -149,6 +150,68 @@ bool peak_order(const gf_peak& l, const gf_peak& r) {
   return better_dm(l, r);
 }
 
+// Sorts long peak lists by (first key, index) on several host threads: each sorts
+// a run, runs are merged pairwise, and the 96-byte records move once.  key(l) <
+// key(r) must mean order(l, r); only equal keys look at the records.  `order` is
+// total up to equal records, so the list is the one std::sort leaves.  Below kParallelPeaks a
+// thread costs more than it saves; kSortThreads keeps several callers (batched
+// searches finish observations side by side) within a host's cores.
+constexpr uint64_t kParallelPeaks = 1 << 14;
+constexpr unsigned kSortThreads = 8;
+
+template <typename Order, typename Key>
+void sort_peak_list(gf_peak* peaks, uint64_t n, Order order, Key key) {
+  unsigned runs = 1;
+  while (2 * runs <= std::min(kSortThreads, std::max(1u, std::thread::hardware_concurrency())) &&
+         n / (2 * runs) >= kParallelPeaks / 4)
+    runs *= 2;
+  if (n < kParallelPeaks || n > std::numeric_limits<uint32_t>::max() || runs == 1) {
+    std::sort(peaks, peaks + n, order);
+    return;
+  }
+  struct Item {
+    double key;
+    uint32_t index;
+  };
+  std::vector<Item> items(n), merged(n);
+  auto less = [&](const Item& x, const Item& y) {
+    if (x.key < y.key) return true;
+    if (y.key < x.key) return false;
+    return order(peaks[x.index], peaks[y.index]);
+  };
+  auto at = [&](uint64_t run) { return static_cast<ptrdiff_t>(n * run / runs); };
+  // calls f(0) .. f(count - 1), each on a thread of its own where one starts
+  auto parallel = [](unsigned count, auto f) {
+    std::vector<std::thread> threads;
+    threads.reserve(count);
+    unsigned k = 1;
+    try {
+      for (; k < count; ++k) threads.emplace_back(f, k);
+    } catch (...) {  // no more threads: the caller does the rest
+    }
+    f(0u);
+    for (unsigned rest = k; rest < count; ++rest) f(rest);
+    for (auto& t : threads) t.join();
+  };
+  parallel(runs, [&](unsigned k) {
+    for (ptrdiff_t i = at(k); i < at(k + 1); ++i) items[i] = Item{key(peaks[i]), static_cast<uint32_t>(i)};
+    std::sort(items.begin() + at(k), items.begin() + at(k + 1), less);
+  });
+  for (unsigned width = 1; width < runs; width *= 2) {
+    parallel(runs / (2 * width), [&](unsigned k) {
+      const uint64_t first = 2ull * width * k;
+      std::merge(items.begin() + at(first), items.begin() + at(first + width), items.begin() + at(first + width),
+                 items.begin() + at(first + 2 * width), merged.begin() + at(first), less);
+    });
+    items.swap(merged);
+  }
+  std::vector<gf_peak> sorted(n);
+  parallel(runs, [&](unsigned k) {
+    for (ptrdiff_t i = at(k); i < at(k + 1); ++i) sorted[i] = peaks[items[i].index];
+  });
+  parallel(runs, [&](unsigned k) { std::copy(sorted.begin() + at(k), sorted.begin() + at(k + 1), peaks + at(k)); });
+}
+
 bool dm_group_order(const gf_peak& l, const gf_peak& r) {
   if (l.dm_index != r.dm_index) return l.dm_index < r.dm_index;
   if (l.width != r.width) return l.width < r.width;
@@ -246,9 +309,9 @@ extern "C" const char* gf_status_string(int status) {
 }
 
 extern "C" const char* gf_build_info(void) {
-  return "gaffa_b200: sm_100a; kernels: stage_kernel, dedisperse_bytes_kernel, subband_stage2_u32_kernel, "
-         "scrunch_kernel, running_median_kernel, detrend_kernel, stats_kernel, normalise_kernel, "
-         "prepare_kernel, ffa_small_kernel, ffa_cluster_kernel, ffa_level_kernel, fold_partial_kernel, "
+  return "gaffa_b200: sm_100a; kernels: stage_kernel, stage_words_kernel, dedisperse_bytes_kernel, "
+         "dedisperse_mma_kernel, subband_stage2_u32_kernel, scrunch_kernel, running_median_kernel, detrend_kernel, "
+         "stats_kernel, normalise_kernel, prepare_kernel, ffa_search_kernel, ffa_level_kernel, fold_partial_kernel, "
          "fold_reduce_kernel, synth_kernel";
 }
 
@@ -296,7 +359,10 @@ extern "C" int gf_make_riptide_ffa_plan(uint64_t nsamples, double tsamp, const g
 extern "C" int gf_sort_peaks(gf_peak* peaks, uint64_t n) {
   return guarded([&] {
     check_arg(n == 0 || peaks, "null argument");
-    std::sort(peaks, peaks + n, better_dm);
+    // finite peaks first, by falling S/N
+    sort_peak_list(peaks, n, better_dm, [](const gf_peak& p) {
+      return finite_peak(p) ? -static_cast<double>(p.snr) : std::numeric_limits<double>::infinity();
+    });
   });
 }
 
@@ -315,7 +381,7 @@ extern "C" int gf_select_candidates(const gf_peak* peaks, uint64_t n, double tob
       check_arg(std::isfinite(p.dm) && std::isfinite(p.period) && std::isfinite(p.frequency) &&
                     std::isfinite(p.duty_cycle) && std::isfinite(p.snr),
                 "Candidate selection peaks must contain finite scientific values");
-    std::sort(sorted.begin(), sorted.end(), peak_order);
+    sort_peak_list(sorted.data(), sorted.size(), peak_order, [](const gf_peak& p) { return p.frequency; });
     const double radius = o->frequency_cluster_radius / tobs;
     std::vector<gf_candidate> cands;
     gf_peak* fb = sorted.data();
