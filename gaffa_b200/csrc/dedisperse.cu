@@ -37,6 +37,7 @@
 // realigning class s by s bytes with one lane shuffle.  Lanes read
 // consecutive words, so every LDS.32 is conflict-free.
 #include "common.cuh"
+#include "mbarrier.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -66,12 +67,7 @@ constexpr int kWords = 8;                       // input words per lane
 constexpr int kOutWords = 32 * kWords - 4;      // 252 output words per warp
 constexpr int kWarpSamples = 4 * kOutWords;     // 1008 samples per warp
 constexpr int kFlushChannels = 256;             // 16-bit lanes hold 256 x 255
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxStages = 4;
-// A stage whose copies have not landed after this many SM cycles (~2 s) is
-// given up: the CTA sets GF_STATUS_PIPELINE in the program's status word
-// (read by gf_dedisp_check) and returns.
-constexpr long long kWaitCycles = 4000000000ll;
 
 struct BytesParams {
   const uint8_t* in;         // group 0, row 0 of the launch
@@ -204,46 +200,8 @@ __device__ __forceinline__ void accumulate_entries(const uint32_t* __restrict__ 
   }
 }
 
-// -- copy ring primitives (PTX ISA 8.x: mbarrier, cp.async.bulk) -------------
+// -- copy ring -------------------------------------------------------------------
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b64 state;\n\t"
-      "mbarrier.arrive.release.cta.shared::cta.b64 state, [%0];\n}\n" ::"r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-// Global -> shared copy of `bytes` (a multiple of 16, both addresses 16-byte
-// aligned) completing on `bar`.  No multicast: the source is this GPU's memory.
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
 __device__ __forceinline__ uint32_t release_stage(uint32_t* counter) {
   uint32_t old;
   asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;\n" : "=r"(old) : "r"(smem_u32(counter)) : "memory");
@@ -438,7 +396,7 @@ __device__ __forceinline__ void bytes_cta(const BytesParams& p, unsigned bx, int
       atomicOr(p.status, GF_STATUS_PIPELINE);
     }
     const long long start = clock64();
-    while (!mbar_try_wait(&ps.full[s], parity) && clock64() - start < kWaitCycles) {
+    while (!mbar_try_wait(&ps.full[s], parity) && clock64() - start < kDrainCycles) {
     }
     return;
   }

@@ -117,24 +117,6 @@ __device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-// Waits for phase `parity`; false when this CTA or another one of the launch
-// gave up, or after kWaitCycles.
-__device__ __forceinline__ bool mma_wait(uint64_t* bar, uint32_t parity, MmaShared& ms, uint32_t* status) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  for (uint32_t i = 0;; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    bool stop = *reinterpret_cast<const volatile uint32_t*>(&ms.failed) != 0;
-    if ((i & 255u) == 255u) stop |= (*reinterpret_cast<const volatile uint32_t*>(status) & GF_STATUS_PIPELINE) != 0;
-    stop |= clock64() - start > kWaitCycles;
-    if (stop) {
-      *reinterpret_cast<volatile uint32_t*>(&ms.failed) = 1u;
-      atomicOr(status, GF_STATUS_PIPELINE);
-      return false;
-    }
-  }
-}
-
 // smem matrix descriptors without swizzle, K-major: start address and the two
 // strides in units of 16 bytes (K halves, then groups of 8 rows), version 1
 constexpr uint64_t kDescWindow = (1ull << 46) | (static_cast<uint64_t>(128 >> 4) << 32) | (static_cast<uint64_t>(16 >> 4) << 16);
@@ -267,7 +249,7 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
         cur = nxt;
         nxt = k + 32 + lane < rows ? __ldg(base + k + 32 + lane) : 0;
       }
-      if (k >= p.stages && !mma_wait(&ms.done[s], parity, ms, p.status)) break;
+      if (k >= p.stages && !wait_warp(&ms.done[s], parity, &ms.failed, p.status)) break;
       const int32_t b = __shfl_sync(kFull, cur, k & 31);
       mma_load_row(p, ms, smem + s * p.stage_bytes, s, src + static_cast<uint64_t>(k) * p.in_row_stride,
                    t0 + static_cast<uint64_t>(b), rec + static_cast<uint64_t>(k) * kRecord, kRecord);
@@ -277,7 +259,7 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
       // gave up: the copies in flight land in this CTA's memory, so wait (bounded) for them
       const long long start = clock64();
       for (int j = max(0, k - p.stages); j < k; ++j)
-        while (!mbar_try_wait(&ms.landed[j % p.stages], (j / p.stages) & 1) && clock64() - start < kWaitCycles) {
+        while (!mbar_try_wait(&ms.landed[j % p.stages], (j / p.stages) & 1) && clock64() - start < kDrainCycles) {
         }
     }
   } else if (Dense && warp == 1) {
@@ -286,7 +268,8 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
     const uint32_t issue = elect_one();
     const uint32_t base16 = smem_u32(smem) >> 4;
     for (int k = 0; k < rows; ++k) {
-      if (!mma_wait(&ms.landed[s], parity, ms, p.status) || !mma_wait(&ms.built[s], parity, ms, p.status)) break;
+      // written after the window and record had landed: implies `landed`
+      if (!wait_warp(&ms.built[s], parity, &ms.failed, p.status)) break;
       tc_fence_after();
       if (issue) {
         const uint32_t stage16 = base16 + ((s * p.stage_bytes) >> 4);
@@ -310,7 +293,8 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
     const uint32_t issue = elect_one();
     const uint32_t base16 = smem_u32(smem) >> 4;
     for (int k = 0; k < rows; ++k) {
-      if (!mma_wait(&ms.landed[s], parity, ms, p.status) || !mma_wait(&ms.built[s], parity, ms, p.status)) break;
+      // written after the window and record had landed: implies `landed`
+      if (!wait_warp(&ms.built[s], parity, &ms.failed, p.status)) break;
       tc_fence_after();
       const uint32_t stage16 = base16 + ((s * p.stage_bytes) >> 4);
       const uint8_t* rec = smem + s * p.stage_bytes + rec_off;
@@ -356,7 +340,7 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
     uint32_t parity = 0;
     uint4 old = make_uint4(0, 0, 0, 0);  // the stage's previous offsets, a byte per DM
     for (int k = w < p.stages ? w : rows; k < rows; k += p.stages, parity ^= 1u) {
-      if (!mma_wait(&ms.landed[s], parity, ms, p.status)) {
+      if (!wait_warp(&ms.landed[s], parity, &ms.failed, p.status)) {
         ok = false;
         break;
       }
@@ -393,8 +377,8 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
     }
     // epilogue: lane n of the accumulator holds samples 16 n .. 16 n + 15, or,
     // dense, lane 16 dm + r samples 16 n + r in columns n
-    ok = ok && mma_wait(&ms.final_bar, 0, ms, p.status);
-    if (__all_sync(kFull, ok)) {
+    ok = ok && wait_warp(&ms.final_bar, 0, &ms.failed, p.status);
+    if (ok) {
       tc_fence_after();
       const int dm_limit = p.dm_skip + (group + 1 == p.ngroups ? p.dm_count_last : p.dm_count);
       const uint32_t lanes = (warp & 3) * 32;
@@ -437,8 +421,9 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
     // a CTA that gave up waits (bounded) for its steps before it frees TMEM
     if (ms.failed) {
       const long long start = clock64();
-      while (!mbar_try_wait(&ms.final_bar, 0) && clock64() - start < kWaitCycles) {
+      while (!mbar_try_wait(&ms.final_bar, 0) && clock64() - start < kDrainCycles) {
       }
+      __syncwarp();
     }
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kMmaColumns));
