@@ -761,6 +761,7 @@ struct BytesStage {
   // tensor-core path (mma.dms > 0: every launch of this stage takes it)
   MmaShape mma;
   int mma_blocks = 0;
+  int32_t mma_max_base = 0;
   DeviceBlob mma_base_dev, mma_rec_dev;
 
   void build(const std::vector<int32_t>& delays, int ng, int ndg, int rpg, int tr, uint64_t nout, int device,
@@ -780,6 +781,7 @@ struct BytesStage {
                        (mma.steps ? kMmaMinCtasDense : kMmaMinCtasSlices)) {
       const MmaTables t = build_mma_tables(delays, ng, ndg, rpg, tr, mma);
       mma_blocks = t.blocks;
+      mma_max_base = t.max_base;
       mma_base_dev.upload(t.base.data(), t.base.size() * sizeof(int32_t), device);
       mma_rec_dev.upload(t.records.data(), t.records.size(), device);
       return;
@@ -878,6 +880,8 @@ struct BytesStage {
     p.tiles = mma.tiles;
     p.steps = mma.steps;
     p.row_bytes = mma.row_bytes;
+    const uint64_t reach = static_cast<uint64_t>(mma_max_base) + mma.row_bytes;
+    p.whole_end = valid >= reach ? valid - reach + 1 : 0;
     p.stage_bytes = mma.stage_bytes;
     p.stages = mma.stages;
     const int b0 = dm_first / mma.dms;

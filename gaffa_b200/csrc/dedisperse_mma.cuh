@@ -70,6 +70,7 @@ struct MmaParams {
   int dms, tiles;             // D, T
   int steps;                  // dense form: K steps of the widest row (0: slices)
   uint32_t row_bytes;         // window bytes per row
+  uint64_t whole_end;         // windows of tiles that start below this lie inside the valid samples
   uint32_t stage_bytes;
   int stages;
   void* out;
@@ -83,6 +84,7 @@ struct MmaShared {
   uint64_t built[kMmaStages];   // the ones are written
   uint64_t done[kMmaStages];    // the tensor core has read the stage (one commit per issuer)
   uint64_t final_bar;           // every step of the CTA has finished
+  uint32_t valid[kMmaStages];   // bytes of the stage's window below the row's valid end
   uint32_t tmem;
   uint32_t failed;
 };
@@ -125,35 +127,20 @@ constexpr uint64_t kDescOnes = (1ull << 46) | (static_cast<uint64_t>(256 >> 4) <
 constexpr uint32_t kIdesc = (2u << 4) | (8u << 24);
 constexpr uint32_t kIdescDense = kIdesc | (32u << 17);   // N = 256
 
-// Copies channel `row`'s window and record into stage `s` (whole loader warp).
-// Samples past the valid end read as zero: the last bulk bytes end on the
-// last 16-byte boundary, the lanes write the rest.
+// Copies a channel's window and record into stage `s` (whole loader warp).  The
+// bulk copy ends on the last 16-byte word with a valid sample (rows are a
+// multiple of 16 bytes); the scatter warp clears what lies past the valid end.
 __device__ __forceinline__ void mma_load_row(const MmaParams& p, MmaShared& ms, uint8_t* stage, int s, const uint8_t* src,
                                              uint64_t t_row, const uint8_t* rec, uint32_t rec_bytes) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t bulk_end = p.in_valid & ~15ull;
-  const uint32_t nbulk = t_row < bulk_end ? static_cast<uint32_t>(umin64(p.row_bytes, bulk_end - t_row)) : 0u;
-  if (nbulk < p.row_bytes) {
-    for (uint32_t b = nbulk + 16 * lane; b < p.row_bytes; b += 512) {
-      const uint64_t t = t_row + b;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (t < p.in_valid) {
-        uint8_t tmp[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) tmp[q] = (t + q < p.in_valid) ? src[t + q] : 0;
-        memcpy(&v, tmp, 16);
-      }
-      *reinterpret_cast<uint4*>(stage + b) = v;
-    }
-    fence_proxy_async_smem();
-    __syncwarp();
-  }
-  if (lane == 0) {
-    mbar_expect_tx(&ms.landed[s], nbulk + rec_bytes);
-    if (nbulk) bulk_copy(stage, src + t_row, nbulk, &ms.landed[s]);
-    bulk_copy(stage + p.stage_bytes - kMmaRecordArea, rec, rec_bytes, &ms.landed[s]);
-    mbar_arrive(&ms.landed[s]);
-  }
+  if ((threadIdx.x & 31) != 0) return;
+  const uint64_t left = t_row < p.in_valid ? p.in_valid - t_row : 0;
+  const uint32_t valid = static_cast<uint32_t>(umin64(p.row_bytes, left));
+  const uint32_t nbulk = (valid + 15u) & ~15u;   // row_bytes is a multiple of 16
+  ms.valid[s] = valid;
+  mbar_expect_tx(&ms.landed[s], nbulk + rec_bytes);
+  if (nbulk) bulk_copy(stage, src + t_row, nbulk, &ms.landed[s]);
+  bulk_copy(stage + p.stage_bytes - kMmaRecordArea, rec, rec_bytes, &ms.landed[s]);
+  mbar_arrive(&ms.landed[s]);
 }
 
 // Issues the N steps of one channel for tiles [tl0, tl1): straight-line code,
@@ -333,6 +320,7 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
     // Lane l writes rows l, l + 32, ... of B (row dm * 16 + r; its 32 bytes are
     // two runs of 16, 128 bytes apart).
     const int w = warp - 3;
+    const bool ragged = t0 >= p.whole_end;
     bool ok = true;
     const uint32_t row0 = (lane >> 3) * 256 + (lane & 7) * 16;
     const int r = lane & 15;
@@ -346,6 +334,14 @@ __device__ __forceinline__ void mma_cta(const MmaParams& p, unsigned bx, int gro
       }
       uint8_t* stage = smem + s * p.stage_bytes;
       const uint4 rec = *reinterpret_cast<const uint4*>(stage + rec_off);
+      // samples past the row's valid end read as zero (the last tiles in time)
+      const uint32_t valid = ragged ? ms.valid[s] : p.row_bytes;
+      if (valid < p.row_bytes) {
+        const uint32_t words = (valid + 15u) & ~15u;
+        if (valid + lane < words) stage[valid + lane] = 0;
+        for (uint32_t b = words + 16 * lane; b < p.row_bytes; b += 512)
+          *reinterpret_cast<uint4*>(stage + b) = make_uint4(0, 0, 0, 0);
+      }
       uint8_t* B = stage + b_off + row0;
       if (Dense) {
         // whole offsets, 16 bits per DM: step x / 32, byte x % 32
@@ -634,6 +630,7 @@ struct MmaTables {
   std::vector<uint8_t> records;  // [group][block][rows_per_group][record]
   uint64_t base_stride = 0;
   int blocks = 0;
+  int32_t max_base = 0;
 };
 
 MmaTables build_mma_tables(const std::vector<int32_t>& delays, int ngroups, int ndm_group, int rows_per_group,
@@ -652,6 +649,7 @@ MmaTables build_mma_tables(const std::vector<int32_t>& delays, int ngroups, int 
         const int n = std::min(m.dms, ndm_group - b * m.dms);
         const size_t at = (static_cast<size_t>(g) * t.blocks + b) * rows_per_group + row;
         t.base[at] = mma_offsets(delays, g, ndm_group, rows_per_group, row, b * m.dms, n, offs);
+        t.max_base = std::max(t.max_base, t.base[at]);
         uint8_t* rec = t.records.data() + at * record;
         if (m.steps) {
           const uint32_t steps = static_cast<uint32_t>(dense_steps(*std::max_element(offs, offs + n)));

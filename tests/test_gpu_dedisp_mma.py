@@ -94,6 +94,22 @@ def test_subband_sums_match_oracle(port, nbits, sbc, npn, ndm):
         assert np.array_equal(run(prog, raw, npn, ndm - npn), want[npn:])
 
 
+@pytest.mark.parametrize("nbits,nsamples", [(2, 150011), (2, 150016), (8, 150001)])
+def test_rows_read_as_zero_past_their_end(port, nbits, nsamples):
+    """Stage one of the subband path sums windows that reach past the last
+    sample, which must count as zeros whatever the staged row's padding holds."""
+    from gaffa_b200 import core, synth
+    freq, data = observation(96, nsamples, 300.0, 400.0, seed=7, levels=4 if nbits == 2 else 256)
+    raw = synth.pack_2bit(data) if nbits == 2 else data
+    prog = core.DedispersionProgram(freq, nsamples, 1e-3, 0.0, 2.0, 48, nbits=nbits, algorithm="subband",
+                                    subband_channels=16, ndm_per_nominal=4)
+    staged = torch.full((int(prog.info.staged_bytes),), 255, dtype=torch.uint8, device="cuda")
+    got = prog.run(prog.stage(torch.from_numpy(raw).cuda(), out=staged))[:, : prog.nout]
+    prog.check()
+    want = port.dedisperse_subband(data, freq, 0.0, 2.0, 48, float(freq.max()), 1e-3, 16, 4)
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), want)
+
+
 def test_batch_of_both_kernels_matches_single_launches():
     from gaffa_b200 import core
     items, want = [], []
