@@ -9,7 +9,7 @@
 // staged once into channel-major rows (one uint8 row per channel, row stride
 // a multiple of 16 bytes); every DM block reuses it.
 //
-// Kernels.  Large launches run on the tensor cores (dedisperse_mma.cuh); the
+// Kernels.  Large launches run on the tensor cores (dedisperse_mma.cu); the
 // byte kernel below takes small ones and pinned launch shapes.
 //
 // Byte kernel.  One CTA = a block of DB DMs x a time tile; each warp owns one DM and
@@ -37,6 +37,7 @@
 // realigning class s by s bytes with one lane shuffle.  Lanes read
 // consecutive words, so every LDS.32 is conflict-free.
 #include "common.cuh"
+#include "dedisperse_mma.cuh"
 #include "mbarrier.cuh"
 
 #include <algorithm>
@@ -457,14 +458,6 @@ __global__ void __launch_bounds__(kThreads, 2) dedisperse_bytes_batch_kernel(con
   const uint32_t local = s_local;
   bytes_cta<uint32_t>(sp, local % sp.grid_x, static_cast<int>(local / sp.grid_x), smem, ps);
 }
-
-}  // namespace
-}  // namespace gf
-
-#include "dedisperse_mma.cuh"
-
-namespace gf {
-namespace {
 
 // Stage-2 sum over uint32 intermediate rows (subband with 8-bit input, where
 // partial sums exceed a byte): out[dm][t] = sum_b inter[b][t + r(dm, b)].
@@ -917,10 +910,7 @@ struct BytesStage {
     if (mma.dms) {
       const MmaParams p = mma_params(in, row_stride, group_stride, valid, g0, gcount, dm_first, dm_count,
                                      dm_count_last, out, out_row_stride, out_dm_rows, out_group_rows, nout);
-      auto kernel = mma.steps ? dedisperse_mma_kernel<OutT, true> : dedisperse_mma_kernel<OutT, false>;
-      set_max_smem(kernel, kMmaBudget);
-      kernel<<<dim3(p.grid_x, 1u, static_cast<unsigned>(gcount)), kMmaThreads, mma.smem, stream>>>(p);
-      cuda_check(cudaGetLastError(), "dedisperse_mma_kernel launch");
+      launch_mma(p, gcount, mma.smem, sizeof(OutT) == 1, stream);
       return;
     }
     const BytesParams p = params(in, row_stride, group_stride, valid, g0, gcount, dm_first, dm_count,
@@ -1335,11 +1325,8 @@ extern "C" int gf_dedisp_batch_run(gf_dedisp_batch* B, void* stream) {
     for (int form = 0; form < 2; ++form) {
       const gf_dedisp_batch::Mma& m = B->mma[form];
       if (m.items == 0) continue;
-      auto kernel = form ? dedisperse_mma_batch_kernel<true> : dedisperse_mma_batch_kernel<false>;
-      set_max_smem(kernel, kMmaBudget);
-      kernel<<<static_cast<unsigned>(m.blocks), kMmaThreads, m.smem, as_stream(stream)>>>(
-          m.items_d.as<MmaParams>(), m.begin_d.as<uint64_t>(), m.items);
-      cuda_check(cudaGetLastError(), "dedisperse_mma_batch_kernel launch");
+      launch_mma_batch(m.items_d.as<MmaParams>(), m.begin_d.as<uint64_t>(), m.items, m.blocks, m.smem, form == 1,
+                       as_stream(stream));
     }
     if (B->nitems == 0) return;
     set_max_smem(dedisperse_bytes_batch_kernel, kBytesMaxSmem);
