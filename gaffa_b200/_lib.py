@@ -197,6 +197,8 @@ _SIGNATURES = [
     ("gf_ffa_transform", C.c_int, [vp, u64, u64, vp, vp, vp]),
     ("gf_dedisp_batch_create", C.c_int, [C.POINTER(DedispBatchItem), u64, C.POINTER(vp)]),
     ("gf_dedisp_batch_run", C.c_int, [vp, vp]),
+    ("gf_dedisp_batch_items", C.c_int, [vp, C.POINTER(u64)]),
+    ("gf_dedisp_kernels", C.c_int, [vp, u64, u64, C.POINTER(i32), C.POINTER(i32)]),
     ("gf_dedisp_batch_destroy", C.c_int, [vp]),
     ("gf_ffa_batch_create", C.c_int, [C.POINTER(FfaBatchMember), u64, i32, C.POINTER(vp)]),
     ("gf_ffa_batch_member_info", C.c_int, [vp, u64, C.POINTER(FfaMemberInfo)]),

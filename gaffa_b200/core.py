@@ -164,6 +164,17 @@ class DedispersionProgram:
         check(_lib.lib().gf_dedisp_workspace_bytes(self._h, dm_count, C.byref(b)))
         return int(b.value)
 
+    # forms of kernels(): gf_dedisp_kernels
+    BYTES, SLICES, DENSE = 0, 1, 2
+
+    def kernels(self, dm_begin: int = 0, dm_count: int | None = None) -> list:
+        """(form, DMs per CTA) of the kernels that run() launches for a DM range:
+        one, or two for the subband path with 8-bit partial sums."""
+        dm_count = self.ndm - dm_begin if dm_count is None else dm_count
+        form, dms = (_lib.i32 * 2)(), (_lib.i32 * 2)()
+        check(_lib.lib().gf_dedisp_kernels(self._h, dm_begin, dm_count, form, dms))
+        return [(f, d) for f, d in zip(form, dms) if f >= 0]
+
     def stage(self, data, stream=None, out: torch.Tensor | None = None) -> torch.Tensor:
         """Channel-major staging of a time-major input (device tensor, or host
         numpy array / tensor copied through a bounce buffer), into `out` when
@@ -217,8 +228,8 @@ class DedispersionProgram:
 
 class DedispersionBatch:
     """Many brute-force (program, staged input, DM range, output) items of
-    different observations as one kernel launch (gf_dedisp_batch_*).  Device
-    pointers are fixed here, so run() can be captured in a CUDA graph; the
+    different observations as one launch per kernel form (gf_dedisp_batch_*).
+    Device pointers are fixed here, so run() can be captured in a CUDA graph; the
     tensors must stay alive as long as the batch."""
 
     def __init__(self, items):
@@ -245,6 +256,13 @@ class DedispersionBatch:
         with torch.cuda.device(device):
             check(_lib.lib().gf_dedisp_batch_create(arr, len(items), C.byref(h)))
         self._h = h
+
+    @property
+    def items_per_kernel(self) -> list:
+        """Items by DedispersionProgram.BYTES, SLICES, DENSE."""
+        n = (_lib.u64 * 3)()
+        check(_lib.lib().gf_dedisp_batch_items(self._h, n))
+        return [int(x) for x in n]
 
     def run(self, stream=None) -> None:
         with torch.cuda.device(self.device):

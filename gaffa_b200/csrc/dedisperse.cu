@@ -9,8 +9,9 @@
 // staged once into channel-major rows (one uint8 row per channel, row stride
 // a multiple of 16 bytes); every DM block reuses it.
 //
-// Kernels.  Large launches run on the tensor cores (dedisperse_mma.cu); the
-// byte kernel below takes small ones and pinned launch shapes.
+// Kernels.  Launches that fill the GPU run on the tensor cores
+// (dedisperse_mma.cu); the byte kernel below takes the others (KernelCost) and
+// pinned launch shapes.
 //
 // Byte kernel.  One CTA = a block of DB DMs x a time tile; each warp owns one DM and
 // 1008 consecutive output samples (252 output words of 4 samples).  The CTA
@@ -623,7 +624,7 @@ Records build_records(const std::vector<int32_t>& delays, int ngroups, int ndm_g
   // + 64 entries: the last chunk's 16-byte base copy may read past its block
   r.base.assign(static_cast<size_t>(ngroups) * blocks * r.base_stride + 64, 0);
   r.words.assign(static_cast<size_t>(ngroups) * ndm_group * r.nchunks * r.record_words, 0u);
-  std::vector<uint16_t> cls[4];
+  uint16_t cls[4][66];   // chunk_rows <= 64, and one more where a class is odd
   for (int g = 0; g < ngroups; ++g) {
     const int grows = std::min(rows_per_group, total_rows - g * rows_per_group);
     for (int b = 0; b < blocks; ++b) {
@@ -636,7 +637,7 @@ Records build_records(const std::vector<int32_t>& delays, int ngroups, int ndm_g
     for (int dm = 0; dm < ndm_group; ++dm) {
       const int b = dm / dms_per_cta;
       for (int k = 0; k < r.nchunks; ++k) {
-        for (auto& c : cls) c.clear();
+        int n[4] = {0, 0, 0, 0};
         const int row0 = k * chunk_rows;
         const int nrows = std::min(chunk_rows, grows - row0);
         for (int i = 0; i < nrows; ++i) {
@@ -645,22 +646,21 @@ Records build_records(const std::vector<int32_t>& delays, int ngroups, int ndm_g
           const int32_t off = d - r.base[(static_cast<size_t>(g) * blocks + b) * r.base_stride + row];
           r.max_off = std::max(r.max_off, off);
           const int word = i * (row_bytes / 4) + (off >> 2);
-          cls[off & 3].push_back(static_cast<uint16_t>(word));
+          cls[off & 3][n[off & 3]++] = static_cast<uint16_t>(word);
         }
         uint32_t* rec = r.words.data() +
                         ((static_cast<size_t>(g) * ndm_group + dm) * r.nchunks + k) * r.record_words;
         uint32_t counts = 0;
-        std::vector<uint16_t> flat;
+        uint32_t* words = rec + 1;
         for (int s = 0; s < 4; ++s) {
           // the count is the class's channels; an odd class takes a whole
           // word for its last entry (high half unused), so classes start on words
-          counts |= static_cast<uint32_t>(cls[s].size()) << (8 * s);
-          if (cls[s].size() & 1) cls[s].push_back(0);
-          flat.insert(flat.end(), cls[s].begin(), cls[s].end());
+          counts |= static_cast<uint32_t>(n[s]) << (8 * s);
+          if (n[s] & 1) cls[s][n[s]] = 0;
+          for (int i = 0; i < n[s]; i += 2)
+            *words++ = static_cast<uint32_t>(cls[s][i]) | (static_cast<uint32_t>(cls[s][i + 1]) << 16);
         }
         rec[0] = counts;
-        for (size_t i = 0; i + 1 < flat.size(); i += 2)
-          rec[1 + i / 2] = static_cast<uint32_t>(flat[i]) | (static_cast<uint32_t>(flat[i + 1]) << 16);
       }
     }
   }
@@ -675,16 +675,6 @@ void set_max_smem(K kernel, size_t bytes) {
   cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
              "cudaFuncSetAttribute(dedisperse smem)");
 }
-
-// The tensor-core kernel runs where all DMs of the program make at least this
-// many of its CTAs (32768 DM-samples each); fewer leave SMs idle, and the byte
-// kernel's CTAs are a quarter of the size.  Byte kernel's automatic shape over
-// tensor-core kernel, 1100-1700 MHz:
-//   dense, 512 channels, 512 CTAs: 2.2x at DM step 0.25, 2.0x at 0.5;
-//     64 channels, 256 CTAs: 2.0x, 2.0x
-//   slices, 512 channels, 512 CTAs: 1.1-1.4x at DM steps 1-32;
-//     1024 channels: 1.06x at 224 CTAs, 0.98x at 200, 0.91x at 144-160
-constexpr uint64_t kMmaMinCtasDense = 148, kMmaMinCtasSlices = 212;
 
 struct Launch {
   int dms_per_cta = kWarps;
@@ -744,14 +734,49 @@ int max_off_estimate(const std::vector<int32_t>& delays, int ngroups, int ndm_gr
   return mo;
 }
 
-// One bytes-kernel configuration with its device tables: ngroups groups of
+// Which kernel a launch takes: the one that the clocks of its CTAs say is faster.
+// A CTA's row takes `alone` clocks while the CTA has an SM to itself and adds
+// `paired` where two share one; `fixed` clocks a CTA (start, first copies, sums
+// out).  Measured, 220 programs of 8 to 4096 channels, 2^15 to 2^19 samples, DM
+// steps 0.05 to 8, each at 8, 16, 32, 64 and all its DMs: within 0.3 % of the
+// faster kernel on average (worst 18 %, on launches of 16 us).  Against the byte
+// kernel alone: 1.11x, worst 0.9x on such launches.
+struct KernelCost {
+  double alone, paired, fixed;
+};
+constexpr double kSms = 148;
+
+double launch_clocks(const KernelCost& c, uint64_t ctas, int rows) {
+  const double share = static_cast<double>(ctas) / kSms;
+  if (share > 4) return share * (c.paired * rows + c.fixed);   // the last wave counts for little
+  const double waves = std::ceil(share), pairs = std::floor(waves / 2);
+  return (2 * pairs * c.paired + (waves - 2 * pairs) * c.alone) * rows + waves * c.fixed;
+}
+
+// The byte kernel by its staged chunk: 8 warps of 1008 samples.
+KernelCost byte_cost(const Launch& l) {
+  if (l.chunk_rows >= 32) return {264, 170, 1500};
+  if (l.chunk_rows == 16) return {325, 204, 1500};
+  return {460, 290, 1500};
+}
+
+// The tensor-core kernel.  Dense: a row's way through the ring (540 clocks, more
+// with few stages) bounds a CTA by itself, two overlap.  Slices: the issue.
+KernelCost mma_cost(const MmaShape& m) {
+  if (m.steps)
+    return {std::max({540.0, 2600.0 / m.stages, m.clocks}), std::max({310.0, 1600.0 / m.stages, m.clocks}), 4000};
+  return {1.05 * m.clocks, 0.75 * m.clocks, 4000};
+}
+
+// One stage of sums with its device tables: ngroups groups of
 // ndm_group DMs over rows_per_group rows (ragged last group).
 struct BytesStage {
   Launch launch;
   Records rec;
   DeviceBlob base_dev, rec_dev, status_dev;
   int ngroups = 0, ndm_group = 0, rows_per_group = 0, total_rows = 0, blocks = 0;
-  // tensor-core path (mma.dms > 0: every launch of this stage takes it)
+  // tables for the tensor-core kernel too (mma.dms > 0), where launches of all
+  // DMs, alone or in a batch, take it; short ranges of DMs may not (takes_mma)
   MmaShape mma;
   int mma_blocks = 0;
   int32_t mma_max_base = 0;
@@ -770,19 +795,43 @@ struct BytesStage {
     status_dev.upload(&zero, sizeof zero, device);
     // a pinned launch shape is a shape of the byte kernel
     if (!dpc_fix && !cr_fix) mma = choose_mma_shape(delays, ng, ndg, rpg, tr);
-    if (mma.dms && ng * ceil_div(ndg, mma.dms) * ceil_div(nout, static_cast<uint64_t>(mma.tiles) * kMmaTile) >=
-                       (mma.steps ? kMmaMinCtasDense : kMmaMinCtasSlices)) {
+    if (mma.dms && (takes_mma(ng, 0, ndg, nout) || prefers_mma(nout))) {
       const MmaTables t = build_mma_tables(delays, ng, ndg, rpg, tr, mma);
       mma_blocks = t.blocks;
       mma_max_base = t.max_base;
       mma_base_dev.upload(t.base.data(), t.base.size() * sizeof(int32_t), device);
       mma_rec_dev.upload(t.records.data(), t.records.size(), device);
-      return;
+    } else {
+      mma = MmaShape{};
     }
-    mma = MmaShape{};
     rec = build_records(delays, ng, ndg, rpg, tr, launch.dms_per_cta, launch.chunk_rows, launch.row_bytes);
     base_dev.upload(rec.base.data(), rec.base.size() * sizeof(int32_t), device);
     rec_dev.upload(rec.words.data(), rec.words.size() * sizeof(uint32_t), device);
+  }
+
+  // CTAs of a launch over `groups` groups and DMs [dm_first, dm_first + dm_count).
+  uint64_t mma_ctas(int groups, int dm_first, int dm_count, uint64_t nout) const {
+    return groups * ceil_div(static_cast<uint64_t>(dm_first % mma.dms + dm_count), mma.dms) *
+           ceil_div(nout, static_cast<uint64_t>(mma.tiles) * kMmaTile);
+  }
+  uint64_t byte_ctas(int groups, int dm_count, uint64_t nout) const {
+    return groups * ceil_div(static_cast<uint64_t>(dm_count), launch.dms_per_cta) *
+           ceil_div(nout, static_cast<uint64_t>(launch.warps_per_dm) * kWarpSamples);
+  }
+  // The launch by itself ...
+  bool takes_mma(int groups, int dm_first, int dm_count, uint64_t nout) const {
+    return mma.dms && launch_clocks(mma_cost(mma), mma_ctas(groups, dm_first, dm_count, nout), rows_per_group) <
+                          launch_clocks(byte_cost(launch), byte_ctas(groups, dm_count, nout), rows_per_group);
+  }
+  // ... and where other launches fill the GPU with it (of all DMs).
+  bool prefers_mma(uint64_t nout) const { return mma_load(0, ndm_group, nout) < byte_load(ndm_group, nout); }
+  double mma_load(int dm_first, int dm_count, uint64_t nout) const {
+    const KernelCost c = mma_cost(mma);
+    return static_cast<double>(mma_ctas(ngroups, dm_first, dm_count, nout)) * (c.paired * rows_per_group + c.fixed);
+  }
+  double byte_load(int dm_count, uint64_t nout) const {
+    const KernelCost c = byte_cost(launch);
+    return static_cast<double>(byte_ctas(ngroups, dm_count, nout)) * (c.paired * rows_per_group + c.fixed);
   }
 
   // Reads and clears the status word (GF_STATUS_PIPELINE: a launch gave up).
@@ -907,7 +956,7 @@ struct BytesStage {
            int gcount, int dm_first, int dm_count, int dm_count_last, void* out,
            uint64_t out_row_stride, uint64_t out_dm_rows, uint64_t out_group_rows, uint64_t nout,
            cudaStream_t stream) const {
-    if (mma.dms) {
+    if (takes_mma(gcount, dm_first, dm_count, nout)) {
       const MmaParams p = mma_params(in, row_stride, group_stride, valid, g0, gcount, dm_first, dm_count,
                                      dm_count_last, out, out_row_stride, out_dm_rows, out_group_rows, nout);
       launch_mma(p, gcount, mma.smem, sizeof(OutT) == 1, stream);
@@ -1158,6 +1207,20 @@ extern "C" int gf_dedisp_stage_from_host(gf_dedisp_program* P, const void* host_
   });
 }
 
+namespace {
+
+// Nominal DMs [n0, n1) of a DM range, and the block-aligned [nb, ne) of stage 1.
+struct SubbandRange {
+  uint64_t n0, n1, nb, ne;
+};
+SubbandRange subband_range(const gf_dedisp_program& P, uint64_t dm_begin, uint64_t dm_count) {
+  const uint64_t n0 = dm_begin / P.npn, n1 = ceil_div(dm_begin + dm_count, P.npn);
+  const uint64_t dpc1 = P.stage1.launch.dms_per_cta;
+  return {n0, n1, (n0 / dpc1) * dpc1, std::min<uint64_t>(ceil_div(n1, dpc1) * dpc1, P.nnom)};
+}
+
+}  // namespace
+
 extern "C" int gf_dedisp_run(gf_dedisp_program* P, const void* dev_staged, uint64_t dm_begin,
                              uint64_t dm_count, uint32_t* dev_out, uint64_t out_stride,
                              void* dev_workspace, void* stream) {
@@ -1180,14 +1243,10 @@ extern "C" int gf_dedisp_run(gf_dedisp_program* P, const void* dev_staged, uint6
     check_arg(dm_begin % P->npn == 0, "subband dm_begin must be a multiple of ndm_per_nominal");
     check_arg(dm_count % P->npn == 0 || dm_begin + dm_count == d.ndm,
               "subband dm_count must be a multiple of ndm_per_nominal");
-    const uint64_t n0 = dm_begin / P->npn;
-    const uint64_t n1 = ceil_div(dm_begin + dm_count, P->npn);
+    const auto [n0, n1, nb, ne] = subband_range(*P, dm_begin, dm_count);
     // stage 1: nominal DMs [nb, ne) (block aligned) for every subband;
     // workspace row (n - nb) * nsb + b
     const auto& s1 = P->stage1;
-    const uint64_t dpc1 = s1.launch.dms_per_cta;
-    const uint64_t nb = (n0 / dpc1) * dpc1;
-    const uint64_t ne = std::min<uint64_t>(ceil_div(n1, dpc1) * dpc1, P->nnom);
     uint8_t* inter = static_cast<uint8_t*>(dev_workspace);
     const uint64_t elem = P->inter_u8 ? 1 : 4;
     if (P->inter_u8)
@@ -1232,6 +1291,29 @@ extern "C" int gf_dedisp_check(gf_dedisp_program* P, void* stream) {
   });
 }
 
+extern "C" int gf_dedisp_kernels(const gf_dedisp_program* P, uint64_t dm_begin, uint64_t dm_count, int32_t* form,
+                                 int32_t* dms_per_cta) {
+  return guarded([&] {
+    check_arg(P && form && dms_per_cta, "null argument");
+    check_arg(dm_count > 0 && dm_begin < P->desc.ndm && dm_begin + dm_count <= P->desc.ndm, "DM range out of bounds");
+    auto stage = [&](int k, const BytesStage& st, int groups, int first, int count, uint64_t nout) {
+      const bool mma = st.takes_mma(groups, first, count, nout);
+      form[k] = !mma ? GF_DEDISP_KERNEL_BYTES : st.mma.steps ? GF_DEDISP_KERNEL_DENSE : GF_DEDISP_KERNEL_SLICES;
+      dms_per_cta[k] = mma ? st.mma.dms : st.launch.dms_per_cta;
+    };
+    form[1] = GF_DEDISP_KERNEL_NONE;
+    dms_per_cta[1] = 0;
+    if (P->desc.algorithm == GF_DEDISP_BRUTE) {
+      stage(0, P->brute, 1, static_cast<int>(dm_begin), static_cast<int>(dm_count), P->nout);
+      return;
+    }
+    const SubbandRange r = subband_range(*P, dm_begin, dm_count);
+    stage(0, P->stage1, static_cast<int>(P->nsb), static_cast<int>(r.nb), static_cast<int>(r.ne - r.nb),
+          P->inter_len);
+    if (P->inter_u8) stage(1, P->stage2, static_cast<int>(r.n1 - r.n0), 0, static_cast<int>(P->npn), P->nout);
+  });
+}
+
 extern "C" int gf_dedisp_workspace_bytes(const gf_dedisp_program* P, uint64_t dm_count, uint64_t* bytes) {
   return guarded([&] {
     check_arg(P && bytes, "null argument");
@@ -1244,7 +1326,7 @@ extern "C" int gf_dedisp_workspace_bytes(const gf_dedisp_program* P, uint64_t dm
 }
 
 // Batched brute-force dedispersion: the launches of many (program, DM range)
-// items as one grid of dedisperse_bytes_batch_kernel.
+// items as one grid per kernel.
 struct gf_dedisp_batch {
   int device = 0;
   int nitems = 0;
@@ -1260,6 +1342,49 @@ struct gf_dedisp_batch {
   } mma[2];
 };
 
+namespace {
+
+// The form that a batched item would take with the GPU full: -1 the byte
+// kernel, 0 slices, 1 dense.
+int item_form(const gf_dedisp_batch_item& it) {
+  const BytesStage& st = it.program->brute;
+  const uint64_t nout = it.program->nout;
+  const int first = static_cast<int>(it.dm_begin), count = static_cast<int>(it.dm_count);
+  if (!st.mma.dms || st.mma_load(first, count, nout) >= st.byte_load(count, nout)) return -1;
+  return st.mma.steps ? 1 : 0;
+}
+
+// Which forms the batch uses (bit form + 1): a form is a grid of its own, after
+// the others, and pays only where it fills the GPU.  A grid takes its load over
+// the SMs, or its longest CTA's time where that is more.
+int batch_forms(const gf_dedisp_batch_item* items, uint64_t nitems) {
+  int best = 0;
+  double best_clocks = INFINITY;
+  for (int forms = 0; forms < 8; forms += 2) {
+    double load[3] = {0, 0, 0}, longest[3] = {0, 0, 0};
+    for (uint64_t i = 0; i < nitems; ++i) {
+      if (!items[i].program) return 0;  // refused below
+      const BytesStage& st = items[i].program->brute;
+      const int first = static_cast<int>(items[i].dm_begin), count = static_cast<int>(items[i].dm_count);
+      int form = item_form(items[i]);
+      if (!(forms >> (form + 1) & 1)) form = -1;
+      const KernelCost c = form < 0 ? byte_cost(st.launch) : mma_cost(st.mma);
+      load[form + 1] += form < 0 ? st.byte_load(count, items[i].program->nout)
+                                 : st.mma_load(first, count, items[i].program->nout);
+      longest[form + 1] = std::max(longest[form + 1], c.alone * st.rows_per_group + c.fixed);
+    }
+    double clocks = 0;
+    for (int f = 0; f < 3; ++f) clocks += std::max(load[f] / kSms, longest[f]);
+    if (clocks < best_clocks) {
+      best_clocks = clocks;
+      best = forms;
+    }
+  }
+  return best;
+}
+
+}  // namespace
+
 extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_t nitems, gf_dedisp_batch** out) {
   return guarded([&] {
     check_arg(items && out, "null argument");
@@ -1269,6 +1394,7 @@ extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_
     std::vector<BytesParams> params;
     std::vector<MmaParams> mma_params[2];
     std::vector<uint64_t> begin, mma_begin[2];
+    const int forms = batch_forms(items, nitems);
     for (uint64_t i = 0; i < nitems; ++i) {
       const gf_dedisp_batch_item& it = items[i];
       check_arg(it.program && it.dev_staged && it.dev_out, "null argument");
@@ -1281,8 +1407,7 @@ extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_
                 "DM range out of bounds");
       check_arg(it.dm_begin % 8 == 0, "dm_begin must be a multiple of 8");
       check_arg(it.out_stride >= P->nout, "out_stride must be >= nout");
-      if (P->brute.mma.dms) {
-        const int form = P->brute.mma.steps ? 1 : 0;
+      if (const int form = item_form(it); forms >> (form + 1) & 1) {
         mma_params[form].push_back(P->brute.mma_params(static_cast<const uint8_t*>(it.dev_staged), P->row_stride, 0,
                                                        d.nsamples, 0, 1, static_cast<int>(it.dm_begin),
                                                        static_cast<int>(it.dm_count), static_cast<int>(it.dm_count),
@@ -1315,6 +1440,15 @@ extern "C" int gf_dedisp_batch_create(const gf_dedisp_batch_item* items, uint64_
     B->items_d.upload(params.data(), params.size() * sizeof(BytesParams), B->device);
     B->begin_d.upload(begin.data(), begin.size() * sizeof(uint64_t), B->device);
     *out = B.release();
+  });
+}
+
+extern "C" int gf_dedisp_batch_items(const gf_dedisp_batch* B, uint64_t* items) {
+  return guarded([&] {
+    check_arg(B && items, "null argument");
+    items[GF_DEDISP_KERNEL_BYTES] = static_cast<uint64_t>(B->nitems);
+    items[GF_DEDISP_KERNEL_SLICES] = static_cast<uint64_t>(B->mma[0].items);
+    items[GF_DEDISP_KERNEL_DENSE] = static_cast<uint64_t>(B->mma[1].items);
   });
 }
 

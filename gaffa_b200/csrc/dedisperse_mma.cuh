@@ -70,6 +70,7 @@ struct MmaShape {
   uint32_t row_bytes = 0, stage_bytes = 0;
   int stages = 0;
   size_t smem = 0;
+  double clocks = 0;        // estimated tensor-core and shared-memory clocks of a CTA's row
 };
 
 // Clocks of a dense step (128 x 256 x 32 multiply-adds; measured 128.3), and
@@ -107,6 +108,21 @@ int32_t mma_offsets(const std::vector<int32_t>& delays, int group, int ndm_group
   lo &= ~15;
   for (int i = 0; i < n; ++i) offs[i] -= lo;
   return lo;
+}
+
+// The window bases of every row of a (group, DM block), as mma_offsets gives
+// them, in passes along the rows; returns the largest offset.
+int32_t mma_bases(const std::vector<int32_t>& delays, int group, int ndm_group, int rows_per_group, int rows, int d0,
+                  int n, int32_t* base) {
+  const int32_t* d = delays.data() + (static_cast<size_t>(group) * ndm_group + d0) * rows_per_group;
+  std::copy(d, d + rows, base);
+  for (int i = 1; i < n; ++i)
+    for (int row = 0; row < rows; ++row) base[row] = std::min(base[row], d[static_cast<size_t>(i) * rows_per_group + row]);
+  for (int row = 0; row < rows; ++row) base[row] &= ~15;
+  int32_t most = 0;
+  for (int i = 0; i < n; ++i)
+    for (int row = 0; row < rows; ++row) most = std::max(most, d[static_cast<size_t>(i) * rows_per_group + row] - base[row]);
+  return most;
 }
 
 // Tensor-core clocks of one (block, row) step list, plus the shared-memory
@@ -175,7 +191,7 @@ MmaShape choose_mma_shape(const std::vector<int32_t>& delays, int ngroups, int n
   for (int D = kMmaSlots; D >= 1; D >>= 1) {
     const int blocks = static_cast<int>(ceil_div(ndm_group, D));
     const uint64_t pairs = static_cast<uint64_t>(ngroups) * blocks * rows_per_group;
-    const uint64_t step = std::max<uint64_t>(1, pairs / 2048) | 1;
+    const uint64_t step = std::max<uint64_t>(1, pairs / 256) | 1;
     double clocks = 0;
     uint64_t count = 0;
     for (uint64_t i = 0; i < pairs; i += step) {
@@ -195,7 +211,7 @@ MmaShape choose_mma_shape(const std::vector<int32_t>& delays, int ngroups, int n
   {
     const int blocks = static_cast<int>(ceil_div(ndm_group, kDenseDms));
     const uint64_t pairs = static_cast<uint64_t>(ngroups) * blocks * rows_per_group;
-    const uint64_t step = std::max<uint64_t>(1, pairs / 2048) | 1;
+    const uint64_t step = std::max<uint64_t>(1, pairs / 256) | 1;
     double clocks = 0;
     uint64_t count = 0;
     for (uint64_t i = 0; i < pairs; i += step) {
@@ -213,16 +229,16 @@ MmaShape choose_mma_shape(const std::vector<int32_t>& delays, int ngroups, int n
   for (const Option& o : options) {
     if (!std::isfinite(o.clocks)) continue;
     int max_off = 0;
+    std::vector<int32_t> base(rows_per_group);
     const int D = o.D ? o.D : kDenseDms;
     const int blocks = static_cast<int>(ceil_div(ndm_group, D));
     for (int g = 0; g < ngroups; ++g)
       for (int b = 0; b < blocks; ++b)
-        for (int row = 0; row < std::min(rows_per_group, total_rows - g * rows_per_group); ++row) {
-          const int n = std::min(D, ndm_group - b * D);
-          mma_offsets(delays, g, ndm_group, rows_per_group, row, b * D, n, offs);
-          max_off = std::max(max_off, *std::max_element(offs, offs + n));
-        }
-    const MmaShape m = o.D ? mma_shape(o.D, max_off) : dense_shape(max_off);
+        max_off = std::max(max_off, mma_bases(delays, g, ndm_group, rows_per_group,
+                                              std::min(rows_per_group, total_rows - g * rows_per_group), b * D,
+                                              std::min(D, ndm_group - b * D), base.data()));
+    MmaShape m = o.D ? mma_shape(o.D, max_off) : dense_shape(max_off);
+    m.clocks = kMmaSlots * o.clocks;
     if (m.dms) return m;
   }
   return MmaShape{};

@@ -198,6 +198,21 @@ int gf_dedisp_batch_destroy(gf_dedisp_batch* batch);
  * waits (dedispersion_cuda.cu:320-417). */
 int gf_dedisp_check(gf_dedisp_program* program, void* stream);
 
+/* Which kernel gf_dedisp_run launches for DMs [dm_begin, dm_begin + dm_count),
+ * and the DMs of one of its CTAs, in form[0] / dms_per_cta[0]; [1] is stage two
+ * of the subband path (GF_DEDISP_KERNEL_NONE: no such stage, or 32-bit sums). */
+enum {
+  GF_DEDISP_KERNEL_NONE = -1,
+  GF_DEDISP_KERNEL_BYTES = 0,  /* CUDA cores */
+  GF_DEDISP_KERNEL_SLICES = 1, /* tensor cores, a step per distinct delay / 16 */
+  GF_DEDISP_KERNEL_DENSE = 2   /* tensor cores, a step per 32 samples of spread */
+};
+int gf_dedisp_kernels(const gf_dedisp_program* program, uint64_t dm_begin, uint64_t dm_count,
+                      int32_t* form, int32_t* dms_per_cta);
+/* Items of the batch per kernel (by GF_DEDISP_KERNEL_BYTES .. _DENSE); a run
+ * launches one grid for each kernel that has any. */
+int gf_dedisp_batch_items(const gf_dedisp_batch* batch, uint64_t* items);
+
 /* Workspace bytes gf_dedisp_run needs for a batch of dm_count DMs (0 for
  * brute force; the subband intermediate otherwise).  Brute-force batches start
  * at multiples of 8 DMs, subband batches at multiples of ndm_per_nominal. */
