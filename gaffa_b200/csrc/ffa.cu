@@ -40,6 +40,7 @@ namespace {
 
 constexpr int kPrepareThreads = 512;
 constexpr int kPrepareChunk = 16384;
+constexpr size_t kPrepareMaxSmem = 200 * 1024;   // a chunk and the plan's largest downsample factor
 
 struct OctaveDev {
   double factor;          // 1.0 = no downsampling
@@ -838,7 +839,7 @@ PrepareItem prepare_item(const FfaMember& M, const float* dev_series, uint64_t n
   check_arg(dev_series && dev_prepared, "null argument");
   check_arg(nseries > 0 && nseries < (1ull << 31), "nseries out of range");
   check_arg(stride >= M.nsamples, "stride must be >= nsamples");
-  check_arg((kPrepareChunk + M.halo) * sizeof(float) <= 200 * 1024,
+  check_arg((kPrepareChunk + M.halo) * sizeof(float) <= kPrepareMaxSmem,
             "downsample factor too large for the prepare kernel");
   PrepareItem it{};
   it.series = dev_series;
@@ -859,8 +860,9 @@ template <bool Batched>
 void launch_prepare_table(const PrepareTable& tab, uint64_t ctas, uint64_t halo, cudaStream_t s) {
   const size_t smem = (kPrepareChunk + halo) * sizeof(float);
   check_arg(ctas < (1ull << 31), "prepare launch too large");
+  // the same limit for every plan (calls from several threads)
   cuda_check(cudaFuncSetAttribute(prepare_kernel<Batched>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)),
+                                  static_cast<int>(kPrepareMaxSmem)),
              "cudaFuncSetAttribute(prepare_kernel)");
   const dim3 grid(static_cast<unsigned>(ctas), Batched ? 1u : tab.one.nseries);
   prepare_kernel<Batched><<<grid, kPrepareThreads, smem, s>>>(tab);

@@ -92,6 +92,16 @@ __global__ void __launch_bounds__(kThreads) fold_reduce_kernel(const double* __r
 
 uint64_t fold_blocks(uint64_t n) { return ceil_div(n, static_cast<uint64_t>(kThreads) * kSamplesPerThread); }
 
+void launch_fold_partial(const void* dev_input, bool u32, uint64_t n, double step, uint64_t start_sample,
+                         uint64_t nbin, unsigned blocks, double* partial, uint32_t* status, cudaStream_t s) {
+  auto kernel = u32 ? fold_partial_kernel<true> : fold_partial_kernel<false>;
+  // the same limit on every call, whatever its bins (calls from several threads)
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(2 * kMaxBins * sizeof(double))),
+             "cudaFuncSetAttribute(fold)");
+  kernel<<<blocks, kThreads, 2 * nbin * sizeof(double), s>>>(dev_input, n, step, start_sample, nbin, partial, status);
+}
+
 }  // namespace
 }  // namespace gf
 
@@ -121,18 +131,8 @@ extern "C" int gf_fold_time_series(const void* dev_input, int32_t input_is_u32, 
     double* partial = static_cast<double*>(dev_workspace);
     uint32_t* status = reinterpret_cast<uint32_t*>(static_cast<char*>(dev_workspace) + blocks * 2 * nbin * 8);
     cuda_check(cudaMemsetAsync(status, 0, 4, s), "cudaMemsetAsync(fold status)");
-    const size_t smem = 2 * nbin * sizeof(double);
-    if (input_is_u32) {
-      cuda_check(cudaFuncSetAttribute(fold_partial_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)), "cudaFuncSetAttribute(fold)");
-      fold_partial_kernel<true><<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(
-          dev_input, n, step, start_sample, nbin, partial, status);
-    } else {
-      cuda_check(cudaFuncSetAttribute(fold_partial_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)), "cudaFuncSetAttribute(fold)");
-      fold_partial_kernel<false><<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(
-          dev_input, n, step, start_sample, nbin, partial, status);
-    }
+    launch_fold_partial(dev_input, input_is_u32 != 0, n, step, start_sample, nbin, static_cast<unsigned>(blocks), partial,
+                        status, s);
     fold_reduce_kernel<<<static_cast<unsigned>(ceil_div(nbin, kThreads)), kThreads, 0, s>>>(
         partial, static_cast<int>(blocks), nbin, dev_profile, dev_exposure);
     cuda_check(cudaGetLastError(), "fold launch");
@@ -215,18 +215,8 @@ extern "C" int gf_fold_time_series_noalloc(const void* dev_input, int32_t input_
     double* partial = static_cast<double*>(fold_scratch_address());
     // the status word must start at zero; the partial sums are overwritten
     cuda_check(cudaMemsetAsync(dev_status, 0, 4, s), "cudaMemsetAsync(fold status)");
-    const size_t smem = 2 * nbin * sizeof(double);
-    if (input_is_u32) {
-      cuda_check(cudaFuncSetAttribute(fold_partial_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)), "cudaFuncSetAttribute(fold)");
-      fold_partial_kernel<true><<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(
-          dev_input, n, step, start_sample, nbin, partial, dev_status);
-    } else {
-      cuda_check(cudaFuncSetAttribute(fold_partial_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)), "cudaFuncSetAttribute(fold)");
-      fold_partial_kernel<false><<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(
-          dev_input, n, step, start_sample, nbin, partial, dev_status);
-    }
+    launch_fold_partial(dev_input, input_is_u32 != 0, n, step, start_sample, nbin, static_cast<unsigned>(blocks), partial,
+                        dev_status, s);
     fold_reduce_kernel<<<static_cast<unsigned>(ceil_div(nbin, kThreads)), kThreads, 0, s>>>(
         partial, static_cast<int>(blocks), nbin, dev_profile, dev_exposure);
     cuda_check(cudaGetLastError(), "fold launch");

@@ -29,6 +29,8 @@ constexpr int kTileT = 64;    // output positions per block
 constexpr int kTileC = 16;    // output channels per block
 constexpr int kMaxCin = 64;
 constexpr int kMaxK = 9;
+// every launch sets the largest layer's limit (calls from several threads)
+constexpr int kConvMaxSmem = static_cast<int>((kMaxCin * (kTileT + kMaxK - 1) + kTileC * kMaxCin * kMaxK) * sizeof(float));
 
 __device__ __forceinline__ float load_f(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ float load_f(const float* p) { return *p; }
@@ -302,7 +304,7 @@ extern "C" int gf_prop_conv_forward(const void* x, const void* w, const float* b
     check_arg(ksize > 0 && ksize <= kMaxK && (ksize & 1), "conv kernel size must be odd and <= 9");
     const size_t smem = (static_cast<size_t>(cin) * (kTileT + ksize - 1) + kTileC * cin * ksize) * sizeof(float);
     auto k = conv_kernel<__nv_bfloat16, __nv_bfloat16>;
-    cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+    cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvMaxSmem),
                "cudaFuncSetAttribute(conv)");
     dim3 grid(static_cast<unsigned>(ceil_div(length, kTileT)), static_cast<unsigned>(ceil_div(cout, kTileC)),
               static_cast<unsigned>(batch));
@@ -331,7 +333,7 @@ extern "C" int gf_prop_conv_backward(const float* dy, const void* y_act, const v
     if (dx) {
       const size_t smem = (static_cast<size_t>(cout) * (kTileT + ksize - 1) + kTileC * cout * ksize) * sizeof(float);
       auto k = conv_kernel<float, float>;
-      cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+      cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvMaxSmem),
                  "cudaFuncSetAttribute(conv)");
       dim3 grid(static_cast<unsigned>(ceil_div(length, kTileT)), static_cast<unsigned>(ceil_div(cin, kTileC)),
                 static_cast<unsigned>(batch));
