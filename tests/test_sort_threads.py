@@ -1,9 +1,14 @@
-"""gf_sort_peaks on lists long enough for several host threads: the order that
-one sort of the whole list gives, at the lengths where the runs change."""
+"""Peak lists long enough for several host threads: the order that one sort of
+the whole list gives, at the lengths where the runs change, and the candidates
+selected from such a list."""
+import os
+
 import numpy as np
 import pytest
 
 from gaffa_b200 import _lib, core
+
+pytestmark = pytest.mark.skipif((os.cpu_count() or 1) < 2, reason="one core: lists are sorted by one thread")
 
 
 def peaks(n, seed):
@@ -32,3 +37,17 @@ def test_long_lists_sort_as_short_ones(n):
         piece = got[a:a + 16000]
         assert np.array_equal(core.sort_peaks(piece[::-1]), piece)
     assert np.array_equal(np.sort(got, order=list(p.dtype.names)), np.sort(p, order=list(p.dtype.names)))
+
+
+@pytest.mark.parametrize("n", [16000, 17200, 40001])   # 2-4 % of them not finite
+def test_candidates_of_long_lists(port, n):
+    p = peaks(n, n + 1)
+    p = p[np.isfinite(p["snr"]) & np.isfinite(p["period"])]   # 49 frequencies: ties decide the order
+    p["duty_cycle"] = 0.1
+    tobs = 300.0
+    for args in ((), (0.5, 3, False, 5)):
+        assert np.array_equal(core.select_candidates(p, tobs, *args), port.select_candidates(p, tobs, *args))
+    # more candidates than the first buffer holds
+    p["period"] = 0.01 + np.arange(len(p)) * 1e-4
+    p["frequency"] = 1.0 / p["period"]
+    assert np.array_equal(core.select_candidates(p, 1e9), port.select_candidates(p, 1e9))
