@@ -8,8 +8,8 @@ FFA period ranges would leave the GPU idle at the tail of every launch.
 Here a batch is cut into pieces (one observation's contiguous DM range) and
 the pieces are packed into waves that fit the series arena.  Each wave runs
 
-* ONE dedispersion launch over all its pieces (gf_dedisp_batch: each CTA
-  finds its piece in a block table),
+* ONE dedispersion launch per kernel form over all its pieces
+  (gf_dedisp_batch: each CTA finds its piece in a block table),
 * ONE launch per preprocessing stage (scrunch, running median, detrend,
   statistics) and ONE FFA-prepare launch over all its pieces
   (gf_preprocess_batch, gf_ffa_batch_prepare_all: item tables likewise; the
@@ -18,9 +18,9 @@ the pieces are packed into waves that fit the series arena.  Each wave runs
   of the wave (gf_ffa_batch: the item runs of all members in one table),
 
 captured once into a CUDA graph and replayed on later runs.  The dedispersion
-launch shapes (DMs per CTA, channel rows per staging step) come from an
-autotuner that times candidate shapes on the observation's own data and
-caches the winners by geometry.  Peaks, candidates and harmonic flags are
+launch shapes (DMs per CTA, channel rows per staging step, or the library's
+choice) come, where one is given, from an autotuner that times candidate
+shapes on the observation's own data and caches the winners by geometry.  Peaks, candidates and harmonic flags are
 identical to searching each observation with its own search.DmSearch (the
 kernels and the arithmetic are the same, only the launch grouping differs);
 the fold of the top candidate agrees to the fold's own tolerance (its FP64
@@ -283,12 +283,12 @@ class BatchSearch:
     @property
     def kernel_launches_per_run(self) -> int:
         """Kernels one run launches in its waves: per wave one dedispersion
-        launch, three or four preprocessing stages (scrunch, running median,
+        launch for each kernel form its pieces take, three or four preprocessing stages (scrunch, running median,
         detrend, statistics) and one prepare over all its pieces, and one
         FFA launch per class; each observation's fold adds three."""
         if not self._built:
             raise RuntimeError("the waves are built by the first run()")
-        return sum(1 + w.pre.kernel_launches + 1 + w.ffa.kernel_launches for w in self.waves)
+        return sum(w.dd.kernel_launches + w.pre.kernel_launches + 1 + w.ffa.kernel_launches for w in self.waves)
 
     def stage(self, filterbanks) -> None:
         """Stages every observation's time-major filterbank (device tensor or

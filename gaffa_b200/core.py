@@ -264,6 +264,10 @@ class DedispersionBatch:
         check(_lib.lib().gf_dedisp_batch_items(self._h, n))
         return [int(x) for x in n]
 
+    @property
+    def kernel_launches(self) -> int:
+        return sum(n > 0 for n in self.items_per_kernel)
+
     def run(self, stream=None) -> None:
         with torch.cuda.device(self.device):
             check(_lib.lib().gf_dedisp_batch_run(self._h, _stream(stream)))

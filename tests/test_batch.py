@@ -288,6 +288,28 @@ def test_batch_search_matches_per_observation_search(tmp_path):
 
 
 @pytest.mark.gpu
+def test_batch_counts_the_kernels_it_launches(tmp_path):
+    """kernel_launches_per_run against the kernels of an eager run's trace (the
+    folds of the candidates, in _finish, apart)."""
+    torch = _cuda()
+    from gaffa_b200 import batch, core
+    cs = small_batch(3, seed=21)
+    for c in cs:
+        c.snr_threshold = 1e6           # no candidates, no folds
+    cs[0].dm_step, cs[0].ndm = 0.05, 96
+    cs[1].dm_step, cs[1].ndm = 40.0, 40
+    data = [core.synth_generate(c.obs) for c in cs]
+    bs = batch.BatchSearch(cs, use_graphs=False)
+    bs.run(data)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        bs.run()
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages() for _ in range(e.count) if "gf::" in e.key]
+    assert len(names) == bs.kernel_launches_per_run, names
+
+
+@pytest.mark.gpu
 def test_batch_search_peak_buffer_growth_and_eager_mode():
     _cuda()
     from gaffa_b200 import batch, core, search
