@@ -78,10 +78,13 @@ def plan_pieces(ndm: list, bytes_per_dm: list, wave_bytes: int, granularity: int
 
 class Autotuner:
     """Picks the brute-force dedispersion launch shape (DMs per CTA, channel
-    rows per staging step) by timing candidate shapes on a block of the
-    observation's highest DMs, and caches the winner by geometry (channels,
-    DM step, log2 length) in memory and, given a path, in a JSON file.  All
-    shapes give the same sums; only the speed differs."""
+    rows per staging step) by timing candidate shapes on the observation's
+    highest DMs, at least `dms` of them and enough to fill the GPU, as the
+    launches of a batch do.  The winner is cached by geometry (channels, band,
+    sampling, DM grid, log2 length) in memory and, given a path, in a JSON
+    file; entries of files from before the library's own choice was a candidate
+    have other keys and are left alone.  All shapes give the same sums; only the
+    speed differs."""
 
     # (0, 0): the library's own choice, the tensor-core kernel where it pays
     SHAPES = ((0, 0), (8, 64), (8, 32), (8, 16), (4, 32), (4, 16), (2, 16))
@@ -95,9 +98,18 @@ class Autotuner:
         self.repeats = repeats
         self.timings = {}
 
+    # DM-samples that fill the GPU with the largest CTAs (two of 32768 per SM), twice
+    FULL = 4 * 148 * 32768
+
     @staticmethod
-    def key(nchans: int, dm_step: float, nsamples: int) -> str:
-        return f"brute-u8/nchans={nchans}/dm_step={dm_step:.4g}/log2_nsamples={round(math.log2(nsamples))}"
+    def key(nchans: int, dm_step: float, nsamples: int, config=None) -> str:
+        """config (configs.SearchConfig): the rest of what the choice depends on."""
+        key = f"brute-u8/nchans={nchans}/dm_step={dm_step:.4g}/log2_nsamples={round(math.log2(nsamples))}"
+        if config is None:
+            return key
+        o = config.obs
+        return (f"{key}/log2_ndm={round(math.log2(config.ndm))}/dm_low={config.dm_low:.3g}"
+                f"/band={o.f_low:.5g}-{o.f_high:.5g}/tsamp={o.tsamp:.4g}/auto")
 
     def save(self) -> None:
         if self.path is not None:
@@ -115,7 +127,7 @@ class Autotuner:
                 prog = make_program(shape)
             except ValueError:
                 continue
-            cnt = min(self.dms, prog.ndm)
+            cnt = min(max(self.dms, -(-self.FULL // prog.nout)), prog.ndm)
             begin = (prog.ndm - cnt) // 8 * 8
             cnt = prog.ndm - begin
             out = torch.empty(cnt * ((prog.nout + 3) // 4 * 4), dtype=torch.int32, device=prog.device)
@@ -187,7 +199,7 @@ class BatchSearch:
             self.plans.append(plan)
             self.strides.append((dd.nout + 3) // 4 * 4)
             self.prep.append(plan.prepared_floats)
-        self._tuned = False
+        self.tuned, self._tuned = {}, False   # programs of tuned shapes, by observation
         per_dm = [4 * (s + p) for s, p in zip(self.strides, self.prep)]
         if wave_bytes is None:
             free = torch.cuda.mem_get_info(self.device)[0]
@@ -210,17 +222,45 @@ class BatchSearch:
     # -- setup --------------------------------------------------------------
 
     def _tune(self) -> None:
-        """Rebuilds each observation's dedispersion program with its tuned
-        launch shape (needs the staged data, so it runs on the first run)."""
+        """Builds each observation's dedispersion program with its tuned launch
+        shape (needs the staged data, so it runs on the first run)."""
         for i, c in enumerate(self.configs):
             o = c.obs
-            key = Autotuner.key(o.nchans, c.dm_step, o.nsamples)
+            key = Autotuner.key(o.nchans, c.dm_step, o.nsamples, c)
 
             def make(shape, o=o, c=c):
                 return core.DedispersionProgram(o.frequencies, o.nsamples, o.tsamp, c.dm_low, c.dm_step, c.ndm,
                                                 device_id=self.device_id, launch_shape=shape)
-            self.dd[i] = make(self.tuner.dedispersion_shape(key, make, self.staged[i]))
+            shape = self.tuner.dedispersion_shape(key, make, self.staged[i])
+            if shape != (0, 0):
+                self.tuned[i] = make(shape)
         self._tuned = True
+
+    def _dedispersion(self, w: _Wave, series) -> core.DedispersionBatch:
+        """The wave's dedispersion: with the tuned programs where that is faster
+        than with the automatic ones alone.  Shapes are tuned one observation at
+        a time; in a wave the forms and shapes share the GPU."""
+        def batch(programs):
+            return core.DedispersionBatch(
+                (programs[pc.obs], self.staged[pc.obs], pc.dm_begin, pc.dm_count, s, self.strides[pc.obs])
+                for pc, s in zip(w.pieces, series))
+
+        auto = batch(self.dd)
+        if not any(pc.obs in self.tuned for pc in w.pieces):
+            return auto
+        tuned = batch([self.tuned.get(i, dd) for i, dd in enumerate(self.dd)])
+
+        def milliseconds(b):
+            b.run()
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(self.tuner.repeats):
+                b.run()
+            end.record()
+            end.synchronize()
+            return start.elapsed_time(end)
+
+        return tuned if milliseconds(tuned) < milliseconds(auto) else auto
 
     def _build_waves(self) -> None:
         arena = self._series_arena
@@ -236,9 +276,7 @@ class BatchSearch:
                 prepared.append(arena.view(torch.float32)[off:off + n].view(pc.dm_count, self.prep[pc.obs]))
                 off += n
             w.series = series
-            w.dd = core.DedispersionBatch(
-                (self.dd[pc.obs], self.staged[pc.obs], pc.dm_begin, pc.dm_count, s, self.strides[pc.obs])
-                for pc, s in zip(w.pieces, series))
+            w.dd = self._dedispersion(w, series)
             w.ffa = core.FfaBatchProgram([(self.plans[pc.obs], pc.dm_count) for pc in w.pieces],
                                          device_id=self.device_id, prepared=prepared, scratch=False)
             # one launch per preprocessing stage and one prepare over every piece
@@ -343,7 +381,7 @@ class BatchSearch:
             t2 = time.perf_counter()
             for pre in self.pre:
                 pre.synchronize()
-            for dd in self.dd:
+            for dd in [*self.dd, *self.tuned.values()]:
                 dd.check()
             results = [f.result() for f in futures]
         t3 = time.perf_counter()

@@ -7,6 +7,7 @@ bit for bit, the per-observation search (search.DmSearch) whose kernels are
 pinned to the reference elsewhere; the dedispersion of a batch is also
 checked against the C restatement directly.
 """
+import dataclasses
 import json
 
 import numpy as np
@@ -72,6 +73,18 @@ def test_autotuner_uses_its_cache(tmp_path):
     def never(shape):
         raise AssertionError("a cached shape must not be re-measured")
     assert t.dedispersion_shape(key, never, None) == (4, 32)
+
+
+def test_autotuner_keys_hold_what_the_choice_depends_on():
+    c = small_batch(1)[0]
+    o = c.obs
+    key = Autotuner.key(o.nchans, c.dm_step, o.nsamples, c)
+    assert key != Autotuner.key(o.nchans, c.dm_step, o.nsamples)   # files of shapes timed without the automatic one
+    for change in (dict(ndm=8 * c.ndm), dict(dm_low=100.0)):
+        assert Autotuner.key(o.nchans, c.dm_step, o.nsamples, dataclasses.replace(c, **change)) != key
+    for change in (dict(f_low=o.f_low / 2), dict(tsamp=2 * o.tsamp)):
+        d = dataclasses.replace(c, obs=dataclasses.replace(o, **change))
+        assert Autotuner.key(o.nchans, c.dm_step, o.nsamples, d) != key
 
 
 # ---------------------------------------------------------------------------
@@ -285,6 +298,41 @@ def test_batch_search_matches_per_observation_search(tmp_path):
         _assert_same_result(a, b)
     assert all(w.graph is not None for w in bs.waves)
     assert json.loads((tmp_path / "tune.json").read_text())
+
+
+@pytest.mark.gpu
+def test_autotuner_times_launches_that_fill_the_gpu():
+    """64 of 256 DMs of 2^16 samples are too few tensor-core CTAs for the GPU;
+    the launches of a batch are not (twice as fast there as any pinned shape)."""
+    torch = _cuda()
+    from gaffa_b200 import batch, core
+    freq = np.linspace(1200.0, 1500.0, 256)
+
+    def make(shape):
+        return core.DedispersionProgram(freq, 1 << 16, 64e-6, 0.0, 0.2, 256, launch_shape=shape)
+
+    staged = torch.zeros(int(make((0, 0)).info.staged_bytes), dtype=torch.uint8, device="cuda")
+    assert batch.Autotuner().dedispersion_shape("k", make, staged) == (0, 0)
+
+
+@pytest.mark.gpu
+def test_a_tuned_wave_is_no_slower_than_the_automatic_one():
+    """Shapes that are poor for the wave (here given, elsewhere picked one
+    observation at a time) are not used where the automatic kernels beat them."""
+    _cuda()
+    from gaffa_b200 import batch, core
+    cs = small_batch(3, seed=11)
+    for c in cs:
+        c.dm_step, c.ndm = 0.1, 96
+    data = [core.synth_generate(c.obs) for c in cs]
+    tuner = batch.Autotuner()
+    for c in cs:
+        tuner.cache[batch.Autotuner.key(c.obs.nchans, c.dm_step, c.obs.nsamples, c)] = [2, 16]
+    bs = batch.BatchSearch(cs, tuner=tuner)
+    got = bs.run(data)
+    assert len(bs.tuned) == 3 and all(w.dd.items_per_kernel[0] == 0 for w in bs.waves)
+    for a, b in zip(got, batch.BatchSearch(cs).run(data)):
+        _assert_same_result(a, b)
 
 
 @pytest.mark.gpu
