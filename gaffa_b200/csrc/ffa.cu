@@ -454,6 +454,12 @@ std::vector<std::vector<MetaEntry>> subtree_levels(uint32_t n) {
   return level;
 }
 
+// Subtrees of fewer rows take one level at a time: n rows make some n / 4 groups,
+// for a CTA of 16 or 32 warps.  Search of 10 series of 2^17 samples at periods of
+// 0.4 to 2.8 s (3 to 23 rows a task): 133 us in groups, 128 with rows below 32
+// one level at a time; below 48, plans of 48-64 bins lose 2 %.
+constexpr uint32_t kGroupRows = 32;
+
 // Schedule of a subtree: the odd level out by itself at the leaves (mostly
 // carries there), then two levels per pass up to the root.
 SubHead build_subtree_schedule(uint32_t n, std::vector<uint4>& meta) {
@@ -462,6 +468,7 @@ SubHead build_subtree_schedule(uint32_t n, std::vector<uint4>& meta) {
   meta.resize(meta.size() + sizeof(SubHead) / 16);
   const auto level = subtree_levels(n);
   int l = static_cast<int>(level.size());
+  while (n < kGroupRows && l > 0) h.pass[h.npasses++] = append_pass(level[--l], meta);
   if (l & 1) h.pass[h.npasses++] = append_pass(level[--l], meta);
   while (l > 0) {
     std::vector<QuadOp> ops;
@@ -738,7 +745,19 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
   }
   if (P->sub_meta.empty()) P->sub_meta.resize(1);
   // tasks, trials, column schedules and classes
-  std::map<std::tuple<int, uint32_t, int>, size_t> class_of;
+  // One launch per NB and CTA size: they run one after another, so tasks too large
+  // for the small tiles join the small CTAs (as subtrees) where they are few.  One
+  // series of 2^20 samples, whose classes used to be kept apart by on-chip and
+  // split tasks too: 295 -> 212 us; 13 series at 48-64 bins with 2 large tasks of
+  // 152: 122 -> 110 us.
+  constexpr double kLargeShare = 0.15;
+  double rows_all[17] = {}, rows_large[17] = {};
+  for (const auto& t : P->tasks) {
+    const uint32_t nb = static_cast<uint32_t>(ceil_div(t.bins, 32));
+    rows_all[nb] += static_cast<double>(t.rows);
+    if (t.rows > P->geo[0][nb].max_rows) rows_large[nb] += static_cast<double>(t.rows);
+  }
+  std::map<std::tuple<uint32_t, int>, size_t> class_of;
   for (uint64_t i = 0; i < P->tasks.size(); ++i) {
     const auto& t = P->tasks[i];
     const uint32_t m = P->task_member[i];
@@ -764,8 +783,7 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
       P->trial_dev.push_back(TrialDev{h, wf / (bf - wf) * h, static_cast<uint32_t>(w), 0u});
     }
     const uint32_t nbt = static_cast<uint32_t>(ceil_div(t.bins, 32));
-    // on chip in a 512-thread CTA when it fits, else the 1024-thread tiles
-    const int gi = t.rows <= P->geo[0][nbt].max_rows ? 0 : 1;
+    const int gi = t.rows <= P->geo[0][nbt].max_rows || rows_large[nbt] < kLargeShare * rows_all[nbt] ? 0 : 1;
     const FfaGeometry& g = P->geo[gi][nbt];
     uint32_t ds = 0;
     while (ceil_div(t.rows, 1ull << ds) > g.max_rows) ++ds;
@@ -775,7 +793,7 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
     P->task_dev.push_back(d);
     const uint32_t nb = static_cast<uint32_t>(ceil_div(t.bins, 32));
     const int threads = gi == 0 ? kSmallThreads : kThreads;
-    const std::tuple<int, uint32_t, int> key{ds == 0 ? 0 : 1, nb, threads};
+    const std::tuple<uint32_t, int> key{nb, threads};
     if (!class_of.count(key)) {
       class_of[key] = P->classes.size();
       P->classes.emplace_back();

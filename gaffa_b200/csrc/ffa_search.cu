@@ -457,8 +457,8 @@ template <int NB, int T>
 __device__ __forceinline__ uint32_t eval_subtree(const SearchParams& p, const float* src, uint32_t n, uint32_t bins, bool root,
                                  uint32_t buf0, uint32_t buf1, char* smeta, const char** meta) {
   const uint2 where = __ldg(reinterpret_cast<const uint2*>(p.sub_head + n));  // offset16, size16
+  load_rows_async<NB, T>(src, n, bins, buf0, p.pitch);  // ahead of what waits for `where`
   stage_schedule<T>(smeta, p.sub_meta + where.x, where.y & 0xffffu);
-  load_rows_async<NB, T>(src, n, bins, buf0, p.pitch);
   cp_async_wait_all();
   __syncthreads();
   const SubHead& head = *reinterpret_cast<const SubHead*>(smeta);
@@ -527,7 +527,7 @@ __device__ __forceinline__ void load_header(ColBlock* dst, const ColBlock* src) 
 // run together.  NB = ceil(bins/32) of every task of the launch.
 template <int NB, int T>
 __global__ void __launch_bounds__(T, T == kSmallThreads ? 2 : 1) ffa_search_kernel(SearchParams p) {
-  __shared__ TrialDev trials[kMaxWidths];
+  __shared__ __align__(16) TrialDev trials[kMaxWidths];
   const uint32_t pitch = p.pitch;
   ColBlock* hdr = reinterpret_cast<ColBlock*>(g_smem);
   char* smeta = reinterpret_cast<char*>(g_smem + 32);
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(T, T == kSmallThreads ? 2 : 1) ffa_search_kern
     const uint32_t bins = t.bins;
     // the item's width trials; every path to detection passes a barrier, and so
     // does the end of the last item's detection
-    for (uint32_t k = threadIdx.x; k < t.ntrials; k += T) trials[k] = p.trials[t.trial_offset + k];
+    for (uint32_t k = threadIdx.x; k < t.ntrials; k += T) cp_async16(trials + k, p.trials + t.trial_offset + k);
     const DetectArgs da = make_detect(p, t, trials, series, task);
     const uint32_t cp_pitch = (bins + t.max_width + 2) | 1u;
     const uint32_t dS = t.split_depth;

@@ -210,7 +210,7 @@ struct SearchParams {
   unsigned long long* counters;
   float* scratch;               // per CTA: scratch_elems0 + scratch_elems1 floats
   uint64_t scratch_elems0, scratch_elems1;
-  uint32_t pitch;               // shared-memory row pitch (max bins | 1)
+  uint32_t pitch;               // shared-memory row pitch ((max bins + 3) | 1)
   uint32_t max_rows;            // rows per shared-memory buffer
   uint32_t front;               // floats before the first row buffer
   uint32_t block_rows;          // output rows of a column block (passes but the last)
