@@ -26,13 +26,17 @@ namespace {
 
 constexpr int kMaxMedianWindow = 2047;
 constexpr int kMedianWarps = 4;
-// Windows up to this many samples are selected per output, longer ones slid
-// along the series: selection costs about 1.3 w warp instructions per output in
-// any number of threads, sliding 0.6 w + 60 in one warp per series, one output
-// after another (0.75 us each at w = 101).
+// Windows up to this many samples may be selected per output, longer ones are
+// slid along the series: selection costs about 1.3 w warp instructions per output
+// in any number of threads (whole CTAs of outputs), sliding 0.6 w + 60 in one warp
+// per series, one output after another (0.8 us each at w = 101, until some
+// kSlideSeries of them fill the GPU).  w = 101, selected against slid: 3000 series
+// of 6666 outputs 5.0 / 5.7 ms, 4096 of 6666 6.8 / 6.6, 20,000 of 333 2.4 / 1.5.
 constexpr int kSelectMaxWindow = 127;
 constexpr int kSelectOutputs = 4 * 32 * kMedianWarps;   // per CTA, four per thread
+constexpr double kSlideSeries = 3700;
 constexpr int kStatsThreads = 256;
+constexpr int kStatsGroup = 4;        // series per CTA of launches of many (stats_group)
 constexpr int kStatsSegment = 16384;  // samples per parallel step
 
 __device__ __forceinline__ float load_sample(const void* base, uint64_t i, bool u32) {
@@ -59,7 +63,9 @@ struct PrepItem {
   int32_t w;            // median window (odd)
   int32_t u32;          // series holds uint32 sums
   int32_t normalise, reject_constant;
-  int32_t reserved;
+  int32_t select;       // median by selection (kSelectMaxWindow)
+  uint32_t group;       // series per CTA of the statistics (the launch's)
+  uint32_t reserved;
 };
 
 enum PrepStage { kScrunch = 0, kMedian, kDetrend, kStats, kStages };
@@ -78,10 +84,10 @@ uint64_t stage_ctas(const PrepItem& it, int stage) {
   switch (stage) {
     case kScrunch: return it.factor > 1 ? ceil_div(it.low_n, 128) * it.nseries : 0;
     case kMedian:
-      return it.w <= kSelectMaxWindow ? ceil_div(it.low_n, kSelectOutputs) * it.nseries
+      return it.select ? ceil_div(it.low_n, kSelectOutputs) * it.nseries
                                       : ceil_div(it.nseries, kMedianWarps);
     case kDetrend: return ceil_div(it.n, 256) * it.nseries;
-    default: return it.nseries;
+    default: return ceil_div(it.nseries, it.group);
   }
 }
 
@@ -337,7 +343,7 @@ __global__ void __launch_bounds__(32 * kMedianWarps) running_median_kernel(const
   extern __shared__ float med_smem[];
   uint32_t local;
   const PrepItem& it = cta_item<Batched>(tab, kMedian, sit, sloc, local);
-  if (it.w <= kSelectMaxWindow) {
+  if (it.select) {
     const uint32_t xblocks = static_cast<uint32_t>(ceil_div(it.low_n, kSelectOutputs));
     select_median(it, local / xblocks, static_cast<uint64_t>(local % xblocks) * kSelectOutputs, keys, extremes);
     return;
@@ -403,11 +409,13 @@ __global__ void __launch_bounds__(256) detrend_kernel(const __grid_constant__ Pr
 //   sum y^2 <= 2^53 u^2 (terms are not negative, so partial sums are smaller),
 //   sum |y| <= sqrt(n sum y^2) <= 2^53 u.
 // From the first segment that fails (many bits per sample, or non-finite ones)
-// warp 0 runs the sequential chain: lanes stream the series into shared memory
+// one warp runs the sequential chain: lanes stream the series into shared memory
 // with cp.async (two chunks in flight), lane 0 adds.
 // Bound: HBM and issue on the parallel path, add latency on the chain.
 // Detrend + normalise of 512 series of 2^18 samples: 4.38 -> 2.64 ms (sliding
-// medians).
+// medians).  Level 2^15 and scatter 2^8 make u = 2^-9 (a trend value below 2^15
+// has it), so sums are parallel up to some 2^19 samples; floats of 24 significant
+// bits take the chain from the start.
 constexpr int kStatsChunk = 1024;  // floats per chunk
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -431,82 +439,108 @@ __device__ __forceinline__ void stats_add(float y, double& sum, double& sq, int&
   sq = __dadd_rn(sq, __dmul_rn(a, a));
 }
 
-template <bool Batched>
+// Series per CTA.  The chain keeps one warp of a CTA at work per series, so many
+// series that will need it share CTAs: 3000 series of 2^15 floats 0.92-1.05 ms four
+// to a CTA, 1.71 ms one to a CTA; 1300 uint32 series of 2^18 samples, whose sums
+// are exact, 0.42 ms one to a CTA, 0.69 ms four.
+bool exact_likely(const PrepItem& it) { return it.u32 && it.n <= (1u << 19); }
+uint32_t stats_group(double series, bool exact) { return exact || series <= 8 * 148 ? 1 : kStatsGroup; }
+
+template <bool Batched, int Group>
 __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_constant__ PrepTable tab) {
   __shared__ PrepItem sit;
   __shared__ uint32_t sloc;
   uint32_t local;
   const PrepItem& it = cta_item<Batched>(tab, kStats, sit, sloc, local);
-  __shared__ __align__(16) float buf[2][kStatsChunk];
+  __shared__ __align__(16) float buf[Group][2][kStatsChunk];
   __shared__ double part_sum[kStatsThreads / 32], part_sq[kStatsThreads / 32];
   __shared__ int part_l[kStatsThreads / 32];
   __shared__ int accepted;
+  __shared__ double group_sum[Group], group_sq[Group];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t s = local;
   const uint64_t n = it.n;
-  const float* row = static_cast<const float*>(it.series) + s * it.stride;
-  // vector loads need 16-byte aligned rows
-  const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
-
-  double sum = 0.0, sq = 0.0;   // thread 0's are the running totals
-  int lowest = 1 << 20;
-  uint64_t done = 0;
-  while (done < n) {
-    const uint32_t len = static_cast<uint32_t>(umin64(kStatsSegment, n - done));
-    const float* x = row + done;
-    double a = 0.0, b = 0.0;
-    int l = 1 << 20;
-    bool bad = false;
-    const uint32_t nvec = aligned ? len / 4 : 0;
-#pragma unroll 4
-    for (uint32_t v = threadIdx.x; v < nvec; v += kStatsThreads) {
-      const float4 y = __ldg(reinterpret_cast<const float4*>(x) + v);
-      stats_add(y.x, a, b, l, bad);
-      stats_add(y.y, a, b, l, bad);
-      stats_add(y.z, a, b, l, bad);
-      stats_add(y.w, a, b, l, bad);
-    }
-    for (uint32_t i = 4 * nvec + threadIdx.x; i < len; i += kStatsThreads) stats_add(x[i], a, b, l, bad);
-    if (bad) l = -1;
+  const uint64_t first = static_cast<uint64_t>(local) * Group;
+  uint64_t group_done[Group];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      a = __dadd_rn(a, __shfl_down_sync(0xffffffffu, a, d));
-      b = __dadd_rn(b, __shfl_down_sync(0xffffffffu, b, d));
-      l = min(l, __shfl_down_sync(0xffffffffu, l, d));
+  for (int g = 0; g < Group; ++g) {
+    const uint64_t s = first + g;
+    group_done[g] = n;
+    if (s >= it.nseries) break;
+    const float* row = static_cast<const float*>(it.series) + s * it.stride;
+    // vector loads need 16-byte aligned rows
+    const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+    double sum = 0.0, sq = 0.0;   // thread 0's are the running totals
+    int lowest = 1 << 20;
+    uint64_t done = 0;
+    while (done < n) {
+      const uint32_t len = static_cast<uint32_t>(umin64(kStatsSegment, n - done));
+      const float* x = row + done;
+      double a = 0.0, b = 0.0;
+      int l = 1 << 20;
+      bool bad = false;
+      const uint32_t nvec = aligned ? len / 4 : 0;
+#pragma unroll 4
+      for (uint32_t v = threadIdx.x; v < nvec; v += kStatsThreads) {
+        const float4 y = __ldg(reinterpret_cast<const float4*>(x) + v);
+        stats_add(y.x, a, b, l, bad);
+        stats_add(y.y, a, b, l, bad);
+        stats_add(y.z, a, b, l, bad);
+        stats_add(y.w, a, b, l, bad);
+      }
+      for (uint32_t i = 4 * nvec + threadIdx.x; i < len; i += kStatsThreads) stats_add(x[i], a, b, l, bad);
+      if (bad) l = -1;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) {
+        a = __dadd_rn(a, __shfl_down_sync(0xffffffffu, a, d));
+        b = __dadd_rn(b, __shfl_down_sync(0xffffffffu, b, d));
+        l = min(l, __shfl_down_sync(0xffffffffu, l, d));
+      }
+      if (lane == 0) {
+        part_sum[warp] = a;
+        part_sq[warp] = b;
+        part_l[warp] = l;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double ns = sum, nq = sq;
+        for (int w = 0; w < kStatsThreads / 32; ++w) {
+          ns = __dadd_rn(ns, part_sum[w]);
+          nq = __dadd_rn(nq, part_sq[w]);
+          lowest = min(lowest, part_l[w]);
+        }
+        bool ok = lowest >= 0;
+        if (ok && lowest < (1 << 20)) {
+          // margins for the rounding of nq itself where it is not exact
+          const int u = lowest - 150;
+          ok = nq <= 0.999 * ldexp(1.0, 53 + 2 * u) &&
+               sqrt(static_cast<double>(done + len) * nq) * 1.001 <= ldexp(1.0, 53 + u);
+        }
+        if (ok) {
+          sum = ns;
+          sq = nq;
+        }
+        accepted = ok ? 1 : 0;
+      }
+      __syncthreads();
+      if (!accepted) break;
+      done += len;
     }
-    if (lane == 0) {
-      part_sum[warp] = a;
-      part_sq[warp] = b;
-      part_l[warp] = l;
-    }
-    __syncthreads();
     if (threadIdx.x == 0) {
-      double ns = sum, nq = sq;
-      for (int w = 0; w < kStatsThreads / 32; ++w) {
-        ns = __dadd_rn(ns, part_sum[w]);
-        nq = __dadd_rn(nq, part_sq[w]);
-        lowest = min(lowest, part_l[w]);
-      }
-      bool ok = lowest >= 0;
-      if (ok && lowest < (1 << 20)) {
-        // margins for the rounding of nq itself where it is not exact
-        const int u = lowest - 150;
-        ok = nq <= 0.999 * ldexp(1.0, 53 + 2 * u) &&
-             sqrt(static_cast<double>(done + len) * nq) * 1.001 <= ldexp(1.0, 53 + u);
-      }
-      if (ok) {
-        sum = ns;
-        sq = nq;
-      }
-      accepted = ok ? 1 : 0;
+      group_sum[g] = sum;
+      group_sq[g] = sq;
     }
-    __syncthreads();
-    if (!accepted) break;
-    done += len;
+    group_done[g] = done;
   }
-  if (warp != 0) return;
-  sum = __shfl_sync(0xffffffffu, sum, 0);
-  sq = __shfl_sync(0xffffffffu, sq, 0);
+  __syncthreads();
+  const uint64_t s = first + warp;
+  if (warp >= Group || s >= it.nseries) return;
+  double sum = group_sum[warp], sq = group_sq[warp];
+  uint64_t done = group_done[0];
+#pragma unroll
+  for (int g = 1; g < Group; ++g)
+    if (warp == g) done = group_done[g];
+  const float* row = static_cast<const float*>(it.series) + s * it.stride;
+  const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   // the rest, if any, in order (done is a multiple of 4)
   const float* rest = row + done;
   const uint64_t nrest = n - done;
@@ -516,7 +550,7 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
     if (c < nchunks) {
       const uint64_t v0 = c * (kStatsChunk / 4);
       for (int v = lane; v < kStatsChunk / 4; v += 32)
-        if (v0 + v < nvec) cp_async16(&buf[c & 1][4 * v], rest + 4 * (v0 + v));
+        if (v0 + v < nvec) cp_async16(&buf[warp][c & 1][4 * v], rest + 4 * (v0 + v));
     }
     cp_async_commit();
   };
@@ -529,7 +563,7 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
       // four samples per vector load, the next vector loaded and the squares
       // formed ahead of the two dependent add chains (same order as one at a
       // time; len is a multiple of 4)
-      const float4* b4 = reinterpret_cast<const float4*>(buf[c & 1]);
+      const float4* b4 = reinterpret_cast<const float4*>(buf[warp][c & 1]);
       const uint32_t nv = static_cast<uint32_t>(umin64(kStatsChunk, nvec * 4 - c * kStatsChunk) / 4);
       float4 nxt = b4[0];
       for (uint32_t v = 0; v < nv; ++v) {
@@ -664,8 +698,14 @@ PrepItem make_item(const gf_preprocess_desc& d, void* dev_series, int32_t input_
   return it;
 }
 
-size_t median_smem(int w) {
-  if (w <= kSelectMaxWindow) return 0;
+// The rule of kSelectMaxWindow for an item of a launch over `series` series.
+bool select_pays(const PrepItem& it, double series) {
+  const double outputs = static_cast<double>(ceil_div(it.low_n, kSelectOutputs) * kSelectOutputs);
+  return it.w <= kSelectMaxWindow && (it.u32 ? 1.3 : 2.4) * it.w * outputs < (0.6 * it.w + 60) * static_cast<double>(it.low_n) *
+                                                                std::max(1.0, kSlideSeries / series);
+}
+
+size_t slide_smem(int w) {
   const int cap = ((w + 31) / 32) * 32;
   return static_cast<size_t>(kMedianWarps) * 2 * cap * sizeof(float);
 }
@@ -674,20 +714,22 @@ size_t median_smem(int w) {
 // ctas[stage] CTAs; a single one with (x blocks, series) grids for scrunch
 // and detrend (ctas[] then holds x blocks, and the series count is the item's).
 template <bool Batched>
-void launch_stages(const PrepTable& tab, const uint64_t (&ctas)[kStages], size_t med_smem, cudaStream_t s) {
+void launch_stages(const PrepTable& tab, const uint64_t (&ctas)[kStages], size_t med_smem, uint32_t group,
+                   cudaStream_t s) {
   for (int st = 0; st < kStages; ++st)
     check_arg(ctas[st] < (1ull << 31), "preprocessing launch too large");
   const unsigned ny = Batched ? 1u : tab.one.nseries;
   // the largest window's limit on every call (calls from several threads)
   cuda_check(cudaFuncSetAttribute(running_median_kernel<Batched>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(median_smem(kMaxMedianWindow))),
+                                  static_cast<int>(slide_smem(kMaxMedianWindow))),
              "cudaFuncSetAttribute(median)");
   if (ctas[kScrunch]) scrunch_kernel<Batched><<<dim3(static_cast<unsigned>(ctas[kScrunch]), ny), 128, 0, s>>>(tab);
   running_median_kernel<Batched><<<static_cast<unsigned>(ctas[kMedian]), 32 * kMedianWarps, med_smem, s>>>(tab);
   cuda_check(cudaGetLastError(), "running median launch");
   detrend_kernel<Batched><<<dim3(static_cast<unsigned>(ctas[kDetrend]), ny), 256, 0, s>>>(tab);
   cuda_check(cudaGetLastError(), "detrend launch");
-  stats_kernel<Batched><<<static_cast<unsigned>(ctas[kStats]), kStatsThreads, 0, s>>>(tab);
+  auto stats = group == 1 ? stats_kernel<Batched, 1> : stats_kernel<Batched, kStatsGroup>;
+  stats<<<static_cast<unsigned>(ctas[kStats]), kStatsThreads, 0, s>>>(tab);
   cuda_check(cudaGetLastError(), "stats launch");
 }
 
@@ -701,10 +743,12 @@ extern "C" int gf_preprocess_inplace(const gf_preprocess_desc* d, void* dev_seri
     PrepTable tab{};
     tab.one = make_item(*d, dev_series, input_is_u32, nseries, stride, dev_workspace, dev_stats, dev_status);
     check_arg(nseries < 65536, "at most 65535 series per call");
+    tab.one.select = select_pays(tab.one, static_cast<double>(nseries));
+    tab.one.group = stats_group(static_cast<double>(nseries), exact_likely(tab.one));
     uint64_t ctas[kStages];
     for (int st = 0; st < kStages; ++st)
       ctas[st] = (st == kScrunch || st == kDetrend) ? stage_xblocks(tab.one, st) : stage_ctas(tab.one, st);
-    launch_stages<false>(tab, ctas, median_smem(tab.one.w), as_stream(stream));
+    launch_stages<false>(tab, ctas, tab.one.select ? 0 : slide_smem(tab.one.w), tab.one.group, as_stream(stream));
   });
 }
 
@@ -715,6 +759,7 @@ struct gf_preprocess_batch {
   int nitems = 0;
   uint64_t ctas[kStages] = {0, 0, 0, 0};
   size_t med_smem = 0;
+  uint32_t group = 1;
   DeviceBlob items_d, begin_d;
 };
 
@@ -729,15 +774,24 @@ extern "C" int gf_preprocess_batch_create(const gf_preprocess_batch_item* items,
     B->nitems = static_cast<int>(nitems);
     std::vector<PrepItem> its;
     std::vector<uint64_t> begin(kStages * nitems);
+    double series = 0;
+    bool exact = true;
     for (uint64_t i = 0; i < nitems; ++i) {
       const gf_preprocess_batch_item& x = items[i];
       check_arg(x.desc != nullptr, "null argument");
       its.push_back(make_item(*x.desc, x.dev_series, x.input_is_u32, x.nseries, x.stride, x.dev_workspace,
                               x.dev_stats, x.dev_status));
-      B->med_smem = std::max(B->med_smem, median_smem(its.back().w));
+      series += static_cast<double>(x.nseries);
+      exact = exact && exact_likely(its.back());
+    }
+    B->group = stats_group(series, exact);
+    for (uint64_t i = 0; i < nitems; ++i) {
+      its[i].select = select_pays(its[i], series);
+      its[i].group = B->group;
+      if (!its[i].select) B->med_smem = std::max(B->med_smem, slide_smem(its[i].w));
       for (int st = 0; st < kStages; ++st) {
         begin[st * nitems + i] = B->ctas[st];
-        B->ctas[st] += stage_ctas(its.back(), st);
+        B->ctas[st] += stage_ctas(its[i], st);
       }
     }
     DeviceGuard dg(device_id);
@@ -755,7 +809,7 @@ extern "C" int gf_preprocess_batch_run(gf_preprocess_batch* B, void* stream) {
     tab.items = B->items_d.as<PrepItem>();
     tab.begin = B->begin_d.as<uint64_t>();
     tab.nitems = B->nitems;
-    launch_stages<true>(tab, B->ctas, B->med_smem, as_stream(stream));
+    launch_stages<true>(tab, B->ctas, B->med_smem, B->group, as_stream(stream));
   });
 }
 

@@ -48,6 +48,62 @@ def test_stats_have_the_sequential_bits(kind, n, stride):
         assert tuple(got) == sequential_stats(row)
 
 
+@pytest.mark.parametrize("nseries", [1184, 1185, 1190, 1203])
+def test_many_series_share_ctas(nseries):
+    """Launches of more than 1184 series of floats take four to a CTA, also where
+    the last CTA has fewer, with sums that are exact, exact part way and never
+    exact side by side; so do batches of that many in all."""
+    from gaffa_b200 import core
+    n = 16384 + 700
+    rng = np.random.default_rng(nseries)
+    x = np.stack([series(("u32", "loud")[k % 2], n, rng) for k in range(8)])[rng.integers(0, 8, nseries)]
+    f = np.stack([series("f32", n, rng) if k % 2 else series("u32", n, rng).astype(np.float32)
+                  for k in range(8)])[rng.integers(0, 8, nseries)]
+    parts = []
+    for data in (x, f):
+        pre = core.PreprocessProgram(n, 1e-3, window_seconds=0.5, min_points=101, max_series=nseries)
+        t = torch.from_numpy(data).cuda()
+        stats = pre.run(t).cpu().numpy()
+        pre.synchronize()
+        y = t.view(torch.float32).cpu().numpy()
+        done = {}
+        for got, row in zip(stats, y):
+            key = row.tobytes()
+            if key not in done:
+                done[key] = sequential_stats(row)
+            assert tuple(got) == done[key]
+        parts.append((data, y, stats))
+    # as two pieces of a batch
+    cut = 600
+    for data, want, want_stats in parts:
+        pres = [core.PreprocessProgram(n, 1e-3, window_seconds=0.5, min_points=101, max_series=m)
+                for m in (cut, nseries - cut)]
+        bufs = [torch.from_numpy(np.ascontiguousarray(d)).cuda() for d in (data[:cut], data[cut:])]
+        core.PreprocessBatch((p, b, b.shape[0]) for p, b in zip(pres, bufs)).run()
+        for p in pres:
+            p.synchronize()
+        assert np.array_equal(np.concatenate([b.view(torch.float32).cpu().numpy() for b in bufs]), want)
+        assert np.array_equal(np.concatenate([p.stats[: b.shape[0]].cpu().numpy() for p, b in zip(pres, bufs)]),
+                              want_stats)
+
+
+@pytest.mark.parametrize("u32", [False, True])
+def test_medians_of_many_series(u32):
+    """Short windows slide where the series fill the GPU: the same medians."""
+    from gaffa_b200 import core
+    rng = np.random.default_rng(4)
+    n, m, w = 700, 5000, 101
+    base = rng.integers(-500, 500, size=(16, n)) + (100000 if u32 else 0)
+    pick = rng.integers(0, 16, m)
+    x = base[pick].astype(np.int32 if u32 else np.float32)
+    t = torch.from_numpy(x).cuda()
+    pre = core.PreprocessProgram(n, 1.0, window_seconds=float(w), min_points=w, max_series=m)
+    pre.run(t)
+    padded = np.pad(base.astype(np.float32), ((0, 0), (w // 2, w // 2)), mode="edge")
+    med = np.median(np.lib.stride_tricks.sliding_window_view(padded, w, axis=1), axis=2).astype(np.float32)
+    assert np.array_equal(t.view(torch.float32).cpu().numpy(), x.astype(np.float32) - med[pick])
+
+
 def test_nonfinite_after_an_exact_segment():
     from gaffa_b200 import core
     x = np.random.default_rng(1).normal(size=(1, 50000)).astype(np.float32)
