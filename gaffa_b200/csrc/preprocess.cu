@@ -457,14 +457,12 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
   __shared__ int part_l[kStatsThreads / 32];
   __shared__ int accepted;
   __shared__ double group_sum[Group], group_sq[Group];
+  __shared__ uint64_t group_done[Group];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t n = it.n;
   const uint64_t first = static_cast<uint64_t>(local) * Group;
-  uint64_t group_done[Group];
-#pragma unroll
   for (int g = 0; g < Group; ++g) {
     const uint64_t s = first + g;
-    group_done[g] = n;
     if (s >= it.nseries) break;
     const float* row = static_cast<const float*>(it.series) + s * it.stride;
     // vector loads need 16-byte aligned rows
@@ -528,17 +526,14 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
     if (threadIdx.x == 0) {
       group_sum[g] = sum;
       group_sq[g] = sq;
+      group_done[g] = done;
     }
-    group_done[g] = done;
   }
   __syncthreads();
   const uint64_t s = first + warp;
   if (warp >= Group || s >= it.nseries) return;
   double sum = group_sum[warp], sq = group_sq[warp];
-  uint64_t done = group_done[0];
-#pragma unroll
-  for (int g = 1; g < Group; ++g)
-    if (warp == g) done = group_done[g];
+  const uint64_t done = group_done[warp];
   const float* row = static_cast<const float*>(it.series) + s * it.stride;
   const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   // the rest, if any, in order (done is a multiple of 4)
