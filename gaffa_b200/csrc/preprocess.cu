@@ -258,8 +258,7 @@ __device__ void slide_median(const PrepItem& it, uint64_t s, float* med_smem) {
 // counts every window from shared memory, one 16-byte load per four samples and
 // four outputs.  Bound: issue, two instructions per comparison.  Detrend +
 // normalise of 512 series whose median runs over 1702 samples, w = 101: 2.64 ->
-// 1.84 ms with it; one 19-DM search of 212 such samples: 3.14 -> 2.44 ms, a
-// ragged second DM batch saved included.
+// 1.84 ms with it.
 __device__ void select_median(const PrepItem& it, uint64_t s, uint64_t i0, uint32_t* keys, uint32_t* extremes) {
   constexpr int kKeys = kSelectOutputs + kSelectMaxWindow + 1;
   const bool scrunched = it.factor > 1;

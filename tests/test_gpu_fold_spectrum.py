@@ -51,4 +51,5 @@ def test_fold_spectrum_and_projections(ns, nc, nbin, sub, period, start, nout, d
     c, ex = cube.cpu().numpy().astype(np.float64), want_e.sum(0)
     ok = ex > 0
     np.testing.assert_allclose(prof.cpu().numpy()[ok], ((c * e).sum((0, 1)) / (k * np.where(ok, ex, 1)))[ok], rtol=1e-6)
+    np.testing.assert_allclose(freq.cpu().numpy(), np.where(ok, (c * e).sum(0) / np.where(ok, ex, 1), 0.0), rtol=1e-6)
     np.testing.assert_allclose(time.cpu().numpy(), np.where(want_e > 0, c.mean(1), 0.0), rtol=1e-6)
