@@ -788,8 +788,13 @@ struct BytesStage {
     ndm_group = ndg;
     rows_per_group = rpg;
     total_rows = tr;
-    launch = choose_launch([&](int dpc) { return max_off_estimate(delays, ng, ndg, rpg, tr, dpc); }, dpc_fix,
-                           cr_fix);
+    int max_off[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};   // by DMs per CTA; asked for with each budget
+    launch = choose_launch(
+        [&](int dpc) {
+          if (max_off[dpc] < 0) max_off[dpc] = max_off_estimate(delays, ng, ndg, rpg, tr, dpc);
+          return max_off[dpc];
+        },
+        dpc_fix, cr_fix);
     blocks = static_cast<int>(ceil_div(ndg, launch.dms_per_cta));
     const uint32_t zero = 0;
     status_dev.upload(&zero, sizeof zero, device);

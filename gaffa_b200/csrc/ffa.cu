@@ -84,8 +84,10 @@ struct PrepareTable {
 
 uint64_t prepare_ctas(const PrepareItem& it) { return ceil_div(it.n, kPrepareChunk) * it.nseries; }
 
+// Three CTAs per SM (66 KB of shared memory each): with 55 registers two, and 787
+// instead of 670 us for 32 series of 2^22 samples.
 template <bool Batched>
-__global__ void __launch_bounds__(kPrepareThreads) prepare_kernel(const __grid_constant__ PrepareTable tab) {
+__global__ void __launch_bounds__(kPrepareThreads, 3) prepare_kernel(const __grid_constant__ PrepareTable tab) {
   extern __shared__ float xs[];
   __shared__ uint64_t kb[32], cnt_prefix[33];
   __shared__ PrepareItem sit;

@@ -529,10 +529,11 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
     }
   }
   __syncthreads();
-  const uint64_t s = first + warp;
+  const uint64_t s = Group == 1 ? first : first + warp;
   if (warp >= Group || s >= it.nseries) return;
   double sum = group_sum[warp], sq = group_sq[warp];
   const uint64_t done = group_done[warp];
+  float(&ring)[2][kStatsChunk] = buf[Group == 1 ? 0 : warp];
   const float* row = static_cast<const float*>(it.series) + s * it.stride;
   const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   // the rest, if any, in order (done is a multiple of 4)
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
     if (c < nchunks) {
       const uint64_t v0 = c * (kStatsChunk / 4);
       for (int v = lane; v < kStatsChunk / 4; v += 32)
-        if (v0 + v < nvec) cp_async16(&buf[warp][c & 1][4 * v], rest + 4 * (v0 + v));
+        if (v0 + v < nvec) cp_async16(&ring[c & 1][4 * v], rest + 4 * (v0 + v));
     }
     cp_async_commit();
   };
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(kStatsThreads) stats_kernel(const __grid_const
       // four samples per vector load, the next vector loaded and the squares
       // formed ahead of the two dependent add chains (same order as one at a
       // time; len is a multiple of 4)
-      const float4* b4 = reinterpret_cast<const float4*>(buf[warp][c & 1]);
+      const float4* b4 = reinterpret_cast<const float4*>(ring[c & 1]);
       const uint32_t nv = static_cast<uint32_t>(umin64(kStatsChunk, nvec * 4 - c * kStatsChunk) / 4);
       float4 nxt = b4[0];
       for (uint32_t v = 0; v < nv; ++v) {
