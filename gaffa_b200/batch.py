@@ -250,15 +250,18 @@ class BatchSearch:
             return auto
         tuned = batch([self.tuned.get(i, dd) for i, dd in enumerate(self.dd)])
 
-        def milliseconds(b):
-            b.run()
+        def timed(b, repeats):
             start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             start.record()
-            for _ in range(self.tuner.repeats):
+            for _ in range(repeats):
                 b.run()
             end.record()
             end.synchronize()
-            return start.elapsed_time(end)
+            return start.elapsed_time(end) / repeats
+
+        def milliseconds(b):
+            ms = timed(b, 1)
+            return ms if ms > 20.0 else timed(b, self.tuner.repeats)   # a short run's first is its warm-up
 
         return tuned if milliseconds(tuned) < milliseconds(auto) else auto
 
