@@ -44,6 +44,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <limits>
 #include <memory>
 #include <vector>
@@ -798,18 +799,25 @@ struct BytesStage {
     blocks = static_cast<int>(ceil_div(ndg, launch.dms_per_cta));
     const uint32_t zero = 0;
     status_dev.upload(&zero, sizeof zero, device);
+    auto byte_records = [&] {
+      return build_records(delays, ng, ndg, rpg, tr, launch.dms_per_cta, launch.chunk_rows, launch.row_bytes);
+    };
     // a pinned launch shape is a shape of the byte kernel
     if (!dpc_fix && !cr_fix) mma = choose_mma_shape(delays, ng, ndg, rpg, tr);
     if (mma.dms && (takes_mma(ng, 0, ndg, nout) || prefers_mma(nout))) {
+      // both kinds of tables; long ones side by side (a million delays take some 4 ms each)
+      auto records = std::async(delays.size() > (1u << 16) ? std::launch::async | std::launch::deferred
+                                                           : std::launch::deferred, byte_records);
       const MmaTables t = build_mma_tables(delays, ng, ndg, rpg, tr, mma);
       mma_blocks = t.blocks;
       mma_max_base = t.max_base;
       mma_base_dev.upload(t.base.data(), t.base.size() * sizeof(int32_t), device);
       mma_rec_dev.upload(t.records.data(), t.records.size(), device);
+      rec = records.get();
     } else {
       mma = MmaShape{};
+      rec = byte_records();
     }
-    rec = build_records(delays, ng, ndg, rpg, tr, launch.dms_per_cta, launch.chunk_rows, launch.row_bytes);
     base_dev.upload(rec.base.data(), rec.base.size() * sizeof(int32_t), device);
     rec_dev.upload(rec.words.data(), rec.words.size() * sizeof(uint32_t), device);
   }
