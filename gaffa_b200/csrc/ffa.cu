@@ -84,10 +84,11 @@ struct PrepareTable {
 
 uint64_t prepare_ctas(const PrepareItem& it) { return ceil_div(it.n, kPrepareChunk) * it.nseries; }
 
-// Three CTAs per SM (66 KB of shared memory each): with 55 registers two, and 787
-// instead of 670 us for 32 series of 2^22 samples.
-template <bool Batched>
-__global__ void __launch_bounds__(kPrepareThreads, 3) prepare_kernel(const __grid_constant__ PrepareTable tab) {
+// Two or three CTAs per SM (66 KB of shared memory each; 55 or 40 registers): three
+// for launches of many waves (32 series of 2^22 samples 673 us, 787 with two), two
+// where that makes a wave fewer or as many (5 of 1.7 x 10^6: 89 us, 103 with three).
+template <bool Batched, int PerSm>
+__global__ void __launch_bounds__(kPrepareThreads, PerSm) prepare_kernel(const __grid_constant__ PrepareTable tab) {
   extern __shared__ float xs[];
   __shared__ uint64_t kb[32], cnt_prefix[33];
   __shared__ PrepareItem sit;
@@ -758,6 +759,8 @@ std::unique_ptr<gf_ffa_program> build_program(const std::vector<MemberSpec>& spe
     const uint32_t nb = static_cast<uint32_t>(ceil_div(t.bins, 32));
     rows_all[nb] += static_cast<double>(t.rows);
     if (t.rows > P->geo[0][nb].max_rows) rows_large[nb] += static_cast<double>(t.rows);
+    // more than one column pass: too long for a small CTA, and twice the scratch
+    if (t.rows > 8ull * P->geo[0][nb].max_rows) rows_large[nb] = INFINITY;
   }
   std::map<std::tuple<uint32_t, int>, size_t> class_of;
   for (uint64_t i = 0; i < P->tasks.size(); ++i) {
@@ -881,11 +884,15 @@ void launch_prepare_table(const PrepareTable& tab, uint64_t ctas, uint64_t halo,
   const size_t smem = (kPrepareChunk + halo) * sizeof(float);
   check_arg(ctas < (1ull << 31), "prepare launch too large");
   // the same limit for every plan (calls from several threads)
-  cuda_check(cudaFuncSetAttribute(prepare_kernel<Batched>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const uint64_t all = ctas * (Batched ? 1u : tab.one.nseries);
+  // a wave of three per SM takes 1.28 times as long as one of two
+  const bool three = 1.28 * static_cast<double>(ceil_div(all, 3 * 148)) < static_cast<double>(ceil_div(all, 2 * 148));
+  auto kernel = three ? prepare_kernel<Batched, 3> : prepare_kernel<Batched, 2>;
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(kPrepareMaxSmem)),
              "cudaFuncSetAttribute(prepare_kernel)");
   const dim3 grid(static_cast<unsigned>(ctas), Batched ? 1u : tab.one.nseries);
-  prepare_kernel<Batched><<<grid, kPrepareThreads, smem, s>>>(tab);
+  kernel<<<grid, kPrepareThreads, smem, s>>>(tab);
   cuda_check(cudaGetLastError(), "prepare_kernel launch");
 }
 
